@@ -35,7 +35,6 @@ constexpr int kSpansPerTile = kSortPlanTile / kSpan;        // 16
 // backward, 2 warps 9.67, 1 warp 8.85 at the same registers, 7.99 with 32 such CTAs per SM.
 constexpr int kSweepWarps = 1;
 constexpr int kSweepThreads = kSweepWarps * 32;
-constexpr int kFinishWarps = 4;
 // positions whose gradient slices are in flight per group (fewer when a lane holds more of a row)
 template <int kC>
 __host__ __device__ constexpr int sweep_loads() {
@@ -600,40 +599,69 @@ __global__ void __launch_bounds__(kSweepThreads, kMinCtas)
   }
 }
 
-// One warp per span whose last run continues to the right: adds the run's pieces in span order --
-// the span's tail slot, then the head slot of every following span up to and including the first
-// one that the run does not pass through -- and updates the row. Group g takes pieces g, g + NG, ...
+// One CTA per tile, one warp per span: a span whose last run continues to the right owns that run. Its
+// warp adds the run's pieces in span order -- the span's tail slot, then the head slot of every
+// following span up to and including the first one that the run does not pass through -- and updates
+// the row. Group g takes pieces g, g + NG, ...
+// A run of more than kAlonePieces pieces (a hot row: 150 000 lookups leave almost 600) would be a chain
+// of memory round trips for one warp, 0.2 ms whatever the rest of the launch does. It reaches past the
+// tile's end, so a tile owns at most one: the tile's sixteen warps share it, each adding a contiguous
+// sixteenth of the pieces, and the first warp adds the sixteen sums in order. (16 tables x 4 M rows,
+// B 65536, Zipf ids, 26.7 M lookups: the training step 2.68 -> 2.56 ms; 26 tables x 1 M rows, B 8192:
+// 0.898 -> 0.877 ms.)
+constexpr int kAlonePieces = 24;
+static_assert(kAlonePieces >= kSpansPerTile, "a run that is shared reaches past its tile's end");
+
 template <typename WT, int GS, int kC>
-__global__ void __launch_bounds__(kFinishWarps * 32)
+__global__ void __launch_bounds__(kSpansPerTile * 32)
     finish_open_runs_kernel(const __grid_constant__ BwdDev p) {
   constexpr int NG = 32 / GS;
   constexpr int quad_w = GS * 4 * static_cast<int>(sizeof(WT));
-  const int lane = threadIdx.x & 31;
+  __shared__ float4 shared_sum[kSpansPerTile][GS * kC];
+  __shared__ uint32_t shared_span, shared_heads;   // the tile's shared run; heads 0: none
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane / GS, gl = lane % GS;
-  const uint32_t span = blockIdx.x * kFinishWarps + (threadIdx.x >> 5);
-  const uint32_t tile = span / kSpansPerTile;
+  const uint32_t tile = blockIdx.x;
   const uint32_t live_tiles = __ldg(p.total_tiles);
   if (tile >= live_tiles) return;
   const uint4 td = __ldg(p.tile_desc + tile);
-  const int s_off = static_cast<int>(span % kSpansPerTile) * kSpan;
-  if (s_off >= static_cast<int>(td.y)) return;
-  if ((p.span_flags[span] & kSpanTailOwner) == 0) return;
-  const int s_count = static_cast<int>(td.y) - s_off < kSpan ? static_cast<int>(td.y) - s_off : kSpan;
+  const int tile_n = static_cast<int>(td.y);
   const int t = static_cast<int>(td.z);
+  const uint32_t my_span = tile * kSpansPerTile + warp;
+  if (threadIdx.x == 0) shared_heads = 0;
+  __syncthreads();
 
   // pieces after the tail slot: one per following span, the last being the first span that is not
   // passed through (flags of spans the run cannot reach are never decisive)
-  const uint32_t span_limit = live_tiles * kSpansPerTile;
+  const bool owner = warp * kSpan < tile_n && (p.span_flags[my_span] & kSpanTailOwner) != 0;
   uint32_t heads = 0;
-  for (uint32_t v = span + 1;; v += 32) {
-    const uint32_t mine = v + lane;
-    const bool through = mine < span_limit && (p.span_flags[mine] & kSpanThrough) != 0;
-    const uint32_t stop = __ballot_sync(kFullMask, !through);
-    if (stop != 0) {
-      heads += __ffs(stop);
-      break;
+  if (owner) {
+    const uint32_t span_limit = live_tiles * kSpansPerTile;
+    constexpr int kAhead = 4;   // 128 flags per step
+    for (uint32_t v = my_span + 1;; v += 32 * kAhead) {
+      uint32_t stop[kAhead];
+      bool through[kAhead];
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const uint32_t mine = v + 32 * k + lane;
+        through[k] = mine < span_limit && (p.span_flags[mine] & kSpanThrough) != 0;
+      }
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) stop[k] = __ballot_sync(kFullMask, !through[k]);
+      bool found = false;
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        if (!found) {
+          heads += stop[k] != 0 ? __ffs(stop[k]) : 32;
+          found = stop[k] != 0;
+        }
+      }
+      if (found) break;
     }
-    heads += 32;
+    if (heads > kAlonePieces && lane == 0) {
+      shared_span = my_span;
+      shared_heads = heads;
+    }
   }
 
   const int D_begin = __ldg(p.D_offsets + t);
@@ -641,69 +669,105 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
   bool on[kC];
   float4 acc[kC];
 #pragma unroll
-  for (int c = 0; c < kC; ++c) {
-    on[c] = (c * GS + gl) * 4 < D;
-    acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  // piece 0 = tail slot of `span`; piece i >= 1 = head slot of span + i. A row looked up 150 000
-  // times leaves almost 600 pieces to one warp, so eight pieces are requested before the first is
-  // added (the additions keep their order).
-  constexpr int kPieces = 8 / kC;
-  const float* lane_base = p.partials + (gl * 4);
-  auto slot_of = [&](uint32_t i) -> int64_t {
-    return i == 0 ? 2 * static_cast<int64_t>(span) + 1 : 2 * static_cast<int64_t>(span + i);
+  for (int c = 0; c < kC; ++c) on[c] = (c * GS + gl) * 4 < D;
+
+  // acc = pieces [first, last) of the run that `span` owns: piece 0 = its tail slot, piece i >= 1 = the
+  // head slot of span + i. Eight pieces are requested before the first is added.
+  const float* lane_base = p.partials + gl * 4;
+  auto sum_pieces = [&](uint32_t span, uint32_t first, uint32_t last) {
+    constexpr int kPieces = 8 / kC;
+#pragma unroll
+    for (int c = 0; c < kC; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t i0 = first + grp; i0 < last; i0 += NG * kPieces) {
+      float4 x[kPieces][kC];
+#pragma unroll
+      for (int u = 0; u < kPieces; ++u) {
+        const uint32_t i = i0 + u * NG;
+        const uint32_t j = i < last ? i : i0;
+        const int64_t slot = j == 0 ? 2 * static_cast<int64_t>(span) + 1 : 2 * static_cast<int64_t>(span + j);
+        const float* src = lane_base + slot * p.max_D;
+#pragma unroll
+        for (int c = 0; c < kC; ++c) {
+          x[u][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (i < last && on[c]) x[u][c] = *reinterpret_cast<const float4*>(src + c * GS * 4);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kPieces; ++u) {
+#pragma unroll
+        for (int c = 0; c < kC; ++c) {
+          acc[c].x += x[u][c].x;
+          acc[c].y += x[u][c].y;
+          acc[c].z += x[u][c].z;
+          acc[c].w += x[u][c].w;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = GS; o < 32; o <<= 1) {
+#pragma unroll
+      for (int c = 0; c < kC; ++c) {
+        acc[c].x += __shfl_xor_sync(kFullMask, acc[c].x, o);
+        acc[c].y += __shfl_xor_sync(kFullMask, acc[c].y, o);
+        acc[c].z += __shfl_xor_sync(kFullMask, acc[c].z, o);
+        acc[c].w += __shfl_xor_sync(kFullMask, acc[c].w, o);
+      }
+    }
   };
-  for (uint32_t i0 = grp; i0 <= heads; i0 += NG * kPieces) {
-    float4 x[kPieces][kC];
+  // updates the row of the run that `span` owns with the gradient in acc
+  auto update_row = [&](uint32_t span) {
+    float sq = sum_squares<kC>(acc);
 #pragma unroll
-    for (int u = 0; u < kPieces; ++u) {
-      const uint32_t i = i0 + u * NG;
-      const float* src = lane_base + slot_of(i <= heads ? i : i0) * p.max_D;
-#pragma unroll
-      for (int c = 0; c < kC; ++c) {
-        x[u][c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i <= heads && on[c]) x[u][c] = *reinterpret_cast<const float4*>(src + c * GS * 4);
-      }
+    for (int o = GS >> 1; o > 0; o >>= 1) sq += __shfl_xor_sync(kFullMask, sq, o);
+    if (sq == 0.f) return;
+    const int s_off = static_cast<int>(span % kSpansPerTile) * kSpan;
+    const int s_count = tile_n - s_off < kSpan ? tile_n - s_off : kSpan;
+    const uint32_t row = __ldg(reinterpret_cast<const uint32_t*>(p.sorted_keys) + td.x + s_off + s_count - 1);
+    char* wrow = p.dev_weights +
+                 (__ldg(p.weights_offsets + t) + static_cast<int64_t>(row) * D) * static_cast<int64_t>(sizeof(WT)) +
+                 gl * 4 * static_cast<int>(sizeof(WT));
+    float* mptr = nullptr;
+    float m_old = 0.f;
+    if (p.optimizer == B200TBE_OPT_ROWWISE_ADAGRAD) {
+      mptr = p.momentum1 + __ldg(p.momentum1_offsets + t) + row;
+      m_old = *mptr;
     }
-#pragma unroll
-    for (int u = 0; u < kPieces; ++u) {
-#pragma unroll
-      for (int c = 0; c < kC; ++c) {
-        acc[c].x += x[u][c].x;
-        acc[c].y += x[u][c].y;
-        acc[c].z += x[u][c].z;
-        acc[c].w += x[u][c].w;
-      }
-    }
-  }
-#pragma unroll
-  for (int o = GS; o < 32; o <<= 1) {
+    typename Quad<WT>::Raw wv[kC];
 #pragma unroll
     for (int c = 0; c < kC; ++c) {
-      acc[c].x += __shfl_xor_sync(kFullMask, acc[c].x, o);
-      acc[c].y += __shfl_xor_sync(kFullMask, acc[c].y, o);
-      acc[c].z += __shfl_xor_sync(kFullMask, acc[c].z, o);
-      acc[c].w += __shfl_xor_sync(kFullMask, acc[c].w, o);
+      wv[c] = Quad<WT>::zero();
+      if (grp == 0 && on[c]) wv[c] = Quad<WT>::load(wrow + c * quad_w);
     }
+    sweep_update<WT, kC>(p, acc, wv, on, sq, m_old, mptr, wrow, 1.f / static_cast<float>(D), quad_w, grp == 0,
+                         gl == 0);
+  };
+
+  if (owner && heads <= kAlonePieces) {
+    sum_pieces(my_span, 0, heads + 1);
+    update_row(my_span);
   }
-  float sq = sum_squares<kC>(acc);
+  __syncthreads();
+  const uint32_t pieces = shared_heads + 1;
+  if (pieces == 1) return;
+  const uint32_t each = (pieces + kSpansPerTile - 1) / kSpansPerTile;
+  const uint32_t first = warp * each < pieces ? warp * each : pieces;
+  sum_pieces(shared_span, first, first + each < pieces ? first + each : pieces);
 #pragma unroll
-  for (int o = GS >> 1; o > 0; o >>= 1) sq += __shfl_xor_sync(kFullMask, sq, o);
-  if (sq == 0.f) return;
-  const uint32_t row = __ldg(reinterpret_cast<const uint32_t*>(p.sorted_keys) + td.x + s_off + s_count - 1);
-  char* wrow = p.dev_weights + (__ldg(p.weights_offsets + t) + static_cast<int64_t>(row) * D) * static_cast<int64_t>(sizeof(WT)) +
-               gl * 4 * static_cast<int>(sizeof(WT));
-  float* mptr = nullptr;
-  float m_old = 0.f;
-  if (p.optimizer == B200TBE_OPT_ROWWISE_ADAGRAD) {
-    mptr = p.momentum1 + __ldg(p.momentum1_offsets + t) + row;
-    m_old = *mptr;
-  }
-  typename Quad<WT>::Raw wv[kC];
+  for (int c = 0; c < kC; ++c)
+    if (grp == 0) shared_sum[warp][c * GS + gl] = acc[c];
+  __syncthreads();
+  if (warp != 0) return;
 #pragma unroll
   for (int c = 0; c < kC; ++c) {
-    wv[c] = Quad<WT>::zero();
-    if (grp == 0 && on[c]) wv[c] = Quad<WT>::load(wrow + c * quad_w);
+    acc[c] = shared_sum[0][c * GS + gl];
+#pragma unroll
+    for (int w = 1; w < kSpansPerTile; ++w) {
+      const float4 x = shared_sum[w][c * GS + gl];
+      acc[c].x += x.x;
+      acc[c].y += x.y;
+      acc[c].z += x.z;
+      acc[c].w += x.w;
+    }
   }
-  sweep_update<WT, kC>(p, acc, wv, on, sq, m_old, mptr, wrow, 1.f / static_cast<float>(D), quad_w, grp == 0, gl == 0);
+  update_row(shared_span);
 }
