@@ -163,16 +163,13 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<KeyT, kRadix>& sm, cons
       const uint32_t with_bit = __ballot_sync(kFullMask, bit);
       peers &= bit ? with_bit : ~with_bit;
     }
-    if (valid) {
-      const int leader = __ffs(peers) - 1;
-      uint32_t before = 0;
-      if (lane == leader) {
-        before = sm.warp_hist[warp][d];
-        sm.warp_hist[warp][d] = static_cast<uint16_t>(before + __popc(peers));
-      }
-      before = __shfl_sync(peers, before, leader);
-      rank[r] = before + __popc(peers & lanemask_lt);
-    }
+    // Every lane reads its digit's counter, then the lowest lane of each digit advances it. (Handing the
+    // value from that lane to its peers with a shuffle over the peers' mask makes the warp run the
+    // shuffle once per distinct digit, twenty-odd times.)
+    const uint32_t before = sm.warp_hist[warp][d];
+    rank[r] = before + __popc(peers & lanemask_lt);
+    __syncwarp();
+    if (valid && (peers & lanemask_lt) == 0) sm.warp_hist[warp][d] = static_cast<uint16_t>(before + __popc(peers));
     __syncwarp();
   }
   __syncthreads();
