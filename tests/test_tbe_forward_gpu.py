@@ -234,3 +234,41 @@ def test_forward_linearity_at_scale():
                               inp.offsets[t * B:t * B + 33] - lo)
     np.testing.assert_allclose(base[:32, t * D:(t + 1) * D].cpu().numpy(), want, rtol=RTOL_FP16,
                                atol=ATOL_FP16)
+
+
+@pytest.mark.parametrize("wdtype,D", [(np.float32, 132), (np.float32, 200), (np.float32, 256), (np.float32, 260),
+                                      (np.float32, 512), (np.float16, 264), (np.float16, 512), (np.float16, 520),
+                                      (np.float16, 1024)])
+@pytest.mark.parametrize("weighted,pooling,idx_dtype,B", [
+    (False, oracle.SUM, np.int64, 37),        # one bag per warp
+    (True, oracle.MEAN, np.int32, 16001),     # groups of two bags, the last group short
+])
+def test_forward_rows_of_513_to_2048_bytes(wdtype, D, weighted, pooling, idx_dtype, B):
+    """A warp per row: rows that end inside, at and just past a lane's vectors, next to tables of narrow rows and
+    of rows that are not whole vectors; empty bags (the last ones too), ids out of range, one with an infinite
+    weight."""
+    rng = workloads.rng_for(230 + D)
+    Ds, rows = [D, 16, D, 20 if wdtype == np.float16 else 64], [500, 80, 33, 60]
+    T = len(Ds)
+    W, wo, Do = helpers.float_tables(rng, rows, Ds, wdtype, -1.0, 1.0)
+    lengths, _, _ = helpers.ragged_bags(rng, T, B, rows, 0, 9 if B > 100 else 70, empty_fraction=0.2)
+    lengths[B - 3:B] = 0
+    lengths[-2:] = 0
+    offsets = np.zeros(T * B + 1, dtype=np.int64)
+    np.cumsum(lengths, out=offsets[1:])
+    indices = np.concatenate([rng.integers(0, rows[t], size=int(offsets[(t + 1) * B] - offsets[t * B]))
+                              for t in range(T)]).astype(np.int64)
+    bad_at = rng.choice(int(offsets[B]), size=20, replace=False)
+    bad, keep = indices.copy(), np.ones(indices.size, dtype=np.float32)
+    bad[bad_at[:10]], bad[bad_at[10:]], keep[bad_at] = rows[0], -1, 0.0
+    psw = rng.random(indices.size).astype(np.float32) if weighted else None
+    given = None if psw is None else psw.copy()
+    if weighted:
+        given[bad_at[0]] = np.inf
+    got, status = _run(W, wo, Do, rows, B, bad, offsets, given, pooling, torch.float32, idx_dtype=idx_dtype)
+    assert status & cabi.DEV_INDEX_OUT_OF_RANGE
+    ty = oracle.FP32 if wdtype == np.float32 else oracle.FP16
+    want = oracle.tbe_forward(W, ty, wo, Do, B, np.where(keep > 0, indices, 0), offsets,
+                              keep if psw is None else psw * keep, pooling)
+    # sums of at most 70 terms of magnitude <= 1 in another order: 70 * 2^-24 of slack
+    np.testing.assert_allclose(got.cpu().numpy(), want, rtol=RTOL_FP32, atol=ATOL_FP32_UNIT)

@@ -407,4 +407,134 @@ __device__ __forceinline__ void pool_float_bags(const BagLaunch<OT>& p, const ch
   while (cur < nb) close_bag();   // bags without lookups at the group's end (or a group without any)
 }
 
+// As pool_float_bags for rows of more than 512 bytes: the whole warp takes a row, lane l holding vectors
+// l, l + 32, ... (kV of them), so a bag closes without any exchange between lanes. A round is kLoads
+// rows, kLoads * kV loads in flight per lane.
+template <typename WT, typename OT, typename IndexT, bool kWeighted, int kV>
+__device__ __forceinline__ void pool_wide_bags(const BagLaunch<OT>& p, const char* table, int row_bytes,
+                                               int64_t num_rows, int64_t col, int64_t bag0, int b0, int nb,
+                                               int lane) {
+  constexpr int kE = Vec16<WT>::kE;
+  constexpr int kLoads = kBagLoads / kV;
+  static_assert(kLoads >= 1 && 32 % kLoads == 0, "a round's ids come from one batch of 32");
+  // lane i: end of bag i relative to the group's first lookup, made monotone and clamped to 31 bits
+  const int64_t begin = load_index<IndexT>(p.offsets, bag0);
+  int my_end = 0;
+  if (lane < nb) {
+    const int64_t e = load_index<IndexT>(p.offsets, bag0 + lane + 1) - begin;
+    my_end = e < 0 ? 0 : (e > kMaxStream ? kMaxStream : static_cast<int>(e));
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int below = __shfl_up_sync(kFullMask, my_end, o);
+    if (lane >= o && below > my_end) my_end = below;
+  }
+  const int total = __shfl_sync(kFullMask, my_end, nb - 1);
+  const IndexT* idx = reinterpret_cast<const IndexT*>(p.indices) + begin;
+  const float* psw = kWeighted ? p.per_sample_weights + begin : nullptr;
+  const int vecs = row_bytes >> 4;
+  const char* lane_base = table + (lane << 4);
+  bool on[kV];
+#pragma unroll
+  for (int k = 0; k < kV; ++k) on[k] = k * 32 + lane < vecs;
+  const int64_t row_limit = num_rows >= 0 ? num_rows : int64_t{0xffffffff};
+  const bool mean = p.pooling_mode == B200TBE_POOL_MEAN;
+  const int rpd = static_cast<int>(p.rows_per_dest);
+
+  float acc[kV][kE];
+#pragma unroll
+  for (int k = 0; k < kV; ++k)
+#pragma unroll
+    for (int e = 0; e < kE; ++e) acc[k][e] = 0.f;
+  int cur = 0;                                              // bag being summed (warp-uniform)
+  int cur_start = 0;
+  int cur_end = __shfl_sync(kFullMask, my_end, 0);
+  int dest = b0 / rpd;
+  int row_in_dest = b0 - dest * rpd;
+  OT* dst = p.outputs[dest] + static_cast<int64_t>(row_in_dest) * p.output_stride + col + lane * kE;
+
+  auto close_bag = [&]() {
+    const int len = cur_end - cur_start;
+    const float scale = (mean && len > 0) ? 1.f / static_cast<float>(len) : 1.f;
+#pragma unroll
+    for (int k = 0; k < kV; ++k) {
+      float r[kE];
+#pragma unroll
+      for (int e = 0; e < kE; ++e) {
+        r[e] = acc[k][e] * scale;
+        acc[k][e] = 0.f;
+      }
+      if (on[k]) {
+#pragma unroll
+        for (int e = 0; e < kE; e += 4) store_pooled<OT, 4>(dst + k * 32 * kE + e, r + e);
+      }
+    }
+    ++cur;
+    cur_start = cur_end;
+    cur_end = __shfl_sync(kFullMask, my_end, cur & 31);
+    dst += p.output_stride;
+    if (++row_in_dest == rpd && cur < nb) {
+      row_in_dest = 0;
+      dst = p.outputs[++dest] + col + lane * kE;
+    }
+  };
+
+  IndexT next_id = 0;
+  float next_w = 1.f;
+  if (lane < total) {
+    next_id = __ldg(idx + lane);
+    if (kWeighted) next_w = __ldg(psw + lane);
+  }
+  for (int c = 0; c < total; c += 32) {
+    const int n = total - c < 32 ? total - c : 32;
+    uint32_t my_row = kNoRow;
+    const float my_w = next_w;
+    if (lane < n) {
+      const int64_t i = static_cast<int64_t>(next_id);
+      if (i < 0 || i >= row_limit) {
+        if (p.status != nullptr) atomicOr(p.status, B200TBE_DEV_INDEX_OUT_OF_RANGE);
+      } else {
+        my_row = static_cast<uint32_t>(i);
+      }
+    }
+    if (c + 32 + lane < total) {
+      next_id = __ldg(idx + c + 32 + lane);
+      if (kWeighted) next_w = __ldg(psw + c + 32 + lane);
+    }
+    for (int j = 0; j < n; j += kLoads) {
+      uint4 x[kLoads][kV];
+      float w[kLoads];
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) {
+        const uint32_t row = __shfl_sync(kFullMask, my_row, j + u);   // kNoRow past the stream's end
+        if (kWeighted) {
+          w[u] = __shfl_sync(kFullMask, my_w, j + u);
+          if (row == kNoRow) w[u] = 0.f;   // whatever its weight, a skipped lookup adds nothing
+        }
+        const char* src = row_address(lane_base, row, static_cast<uint32_t>(row_bytes));
+#pragma unroll
+        for (int k = 0; k < kV; ++k) {
+          x[u][k] = make_uint4(0u, 0u, 0u, 0u);  // +0.0 in either type: adding it changes nothing
+          if (row != kNoRow && on[k]) x[u][k] = ldg_cached16(src + k * 512);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) {
+        if (j + u < n) {
+          while (c + j + u >= cur_end) close_bag();   // the lookup lies in a later bag
+        }
+#pragma unroll
+        for (int k = 0; k < kV; ++k) {
+          if (kWeighted) {
+            Vec16<WT>::fma(acc[k], x[u][k], w[u]);
+          } else {
+            Vec16<WT>::add(acc[k], x[u][k]);
+          }
+        }
+      }
+    }
+  }
+  while (cur < nb) close_bag();
+}
+
 }  // namespace b200tbe

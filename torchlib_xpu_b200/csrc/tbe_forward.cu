@@ -1,8 +1,9 @@
 // TBE pooled forward over fp32 / fp16 tables.
 //
 // Rows of up to 512 bytes (every D <= 128 fp32 / D <= 256 fp16): the register gather of tbe_bags.cuh,
-// one warp per group of bags in a plain grid of one-warp CTAs. Wider rows run on the shared-memory ring
-// engine of tbe_stream.cuh (persistent, one CTA per SM); rows that are not whole aligned 16-byte
+// one warp per group of bags in a plain grid of one-warp CTAs; rows of up to 2048 bytes likewise, a whole
+// warp per row. Wider rows (fp32, D > 512) run on the shared-memory ring engine of tbe_stream.cuh
+// (persistent, one CTA per SM); rows that are not whole aligned 16-byte
 // vectors on a scalar path.
 #include "tbe_bags.cuh"
 
@@ -128,8 +129,49 @@ __global__ void __launch_bounds__(32, kWeighted ? 24 : kBagCtasPerSm)
                                              p.output_col_offset + D_begin, bag0, b0, nb, lane);
 }
 
+// Calls whose widest rows have 513 to 2048 bytes; every table takes the path of its own width. On the ring
+// engine one such table took all tables there, to one CTA per SM and a copy through shared memory (14 fp32
+// tables of 16 to 256 elements, 42 000 weighted bags, 0.63 M lookups: 100 us; 57 us here, 4.0 TB/s of rows).
+// Sums of four vectors per lane and the rows in flight need more than 64 registers: 24 CTAs per SM, 20
+// with sixteen fp16 elements per vector pair or with weights travelling along.
+constexpr int kWideRowBytes = 2048;
+
+template <typename WT, typename OT, typename IndexT, bool kWeighted>
+__global__ void __launch_bounds__(32, sizeof(WT) == 4 && !kWeighted ? 24 : 20)
+    tbe_forward_wide_bags_kernel(const __grid_constant__ FwdParams p) {
+  const int lane = threadIdx.x;
+  const int t = static_cast<int>(blockIdx.x / static_cast<unsigned>(p.groups_per_table));
+  const int b0 = static_cast<int>(blockIdx.x - static_cast<unsigned>(t) * p.groups_per_table) * p.bag_group;
+  const int nb = p.B - b0 < p.bag_group ? p.B - b0 : p.bag_group;
+  const int64_t bag0 = static_cast<int64_t>(t) * p.B + b0;
+  const int D_begin = __ldg(p.D_offsets + t);
+  const int D = __ldg(p.D_offsets + t + 1) - D_begin;
+  const int row_bytes = D * static_cast<int>(sizeof(WT));
+  const char* table = p.dev_weights + __ldg(p.weights_offsets + t) * static_cast<int64_t>(sizeof(WT));
+  const int64_t num_rows = p.rows_per_table ? __ldg(p.rows_per_table + t) : -1;
+  const int64_t col = p.output_col_offset + D_begin;
+  OT* const* outputs = reinterpret_cast<OT* const*>(p.outputs);
+  if ((row_bytes & 15) != 0 || (reinterpret_cast<uintptr_t>(table) & 15) != 0 || row_bytes > kWideRowBytes ||
+      D <= 0) {
+    pool_unit_generic<OT, IndexT>(p.indices, p.offsets, p.per_sample_weights, p.status,
+                                  p.pooling_mode, sizeof(WT) == 4 ? B200TBE_FP32 : B200TBE_FP16,
+                                  table, row_bytes, D, num_rows, outputs, p.output_stride, col,
+                                  p.rows_per_dest, bag0, b0, nb, lane);
+    return;
+  }
+  const BagLaunch<OT> launch{p.indices, p.offsets, p.per_sample_weights, p.status, p.pooling_mode,
+                             outputs, p.output_stride, p.rows_per_dest};
+  if (row_bytes <= 512) {
+    pool_float_bags<WT, OT, IndexT, kWeighted>(launch, table, row_bytes, num_rows, col, bag0, b0, nb, lane);
+  } else if (row_bytes <= 1024) {
+    pool_wide_bags<WT, OT, IndexT, kWeighted, 2>(launch, table, row_bytes, num_rows, col, bag0, b0, nb, lane);
+  } else {
+    pool_wide_bags<WT, OT, IndexT, kWeighted, 4>(launch, table, row_bytes, num_rows, col, bag0, b0, nb, lane);
+  }
+}
+
 template <typename WT, typename OT, typename IndexT>
-int launch_bags(const FwdParams& d0, cudaStream_t stream) {
+int launch_bags(const FwdParams& d0, bool wide, cudaStream_t stream) {
   const int64_t bags = static_cast<int64_t>(d0.T) * d0.B;
   if (bags > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
   FwdParams d = d0;
@@ -137,7 +179,12 @@ int launch_bags(const FwdParams& d0, cudaStream_t stream) {
   d.groups_per_table = (d.B + d.bag_group - 1) / d.bag_group;
   const unsigned grid = static_cast<unsigned>(static_cast<int64_t>(d.T) * d.groups_per_table);
   const bool weighted = d.per_sample_weights != nullptr;
-  if (d.bag_group == 1) {
+  if (wide) {
+    if (weighted)
+      tbe_forward_wide_bags_kernel<WT, OT, IndexT, true><<<grid, 32, 0, stream>>>(d);
+    else
+      tbe_forward_wide_bags_kernel<WT, OT, IndexT, false><<<grid, 32, 0, stream>>>(d);
+  } else if (d.bag_group == 1) {
     if (weighted)
       tbe_forward_bags_kernel<WT, OT, IndexT, true><<<grid, 32, 0, stream>>>(d);
     else
@@ -165,10 +212,9 @@ int launch_one(const FwdParams& d, cudaStream_t stream) {
 
 template <typename WT, typename OT, typename IndexT>
 int launch_forward(const FwdParams& d, int max_D, cudaStream_t stream) {
-  if (static_cast<int64_t>(max_D) * sizeof(WT) <= 512) return launch_bags<WT, OT, IndexT>(d, stream);
-  if (max_D <= 128) return launch_one<WT, OT, IndexT, 1>(d, stream);
-  if (max_D <= 256) return launch_one<WT, OT, IndexT, 2>(d, stream);
-  if (max_D <= 512) return launch_one<WT, OT, IndexT, 4>(d, stream);
+  const int64_t max_row = static_cast<int64_t>(max_D) * sizeof(WT);
+  if (max_row <= 512) return launch_bags<WT, OT, IndexT>(d, false, stream);
+  if (max_row <= kWideRowBytes) return launch_bags<WT, OT, IndexT>(d, true, stream);
   if (max_D <= 1024) return launch_one<WT, OT, IndexT, 8>(d, stream);
   return B200TBE_ERR_UNSUPPORTED;
 }
