@@ -310,3 +310,93 @@ def test_backward_waits_for_the_gradient_event():
     torch.cuda.synchronize()
     np.testing.assert_allclose(dW.float().cpu().numpy(), W_ref.astype(np.float32), rtol=RTOL, atol=ATOL)
     np.testing.assert_allclose(dm.cpu().numpy(), m_ref, rtol=1e-4, atol=1e-6)
+
+
+def _runs_case(rng, runs, D, wdtype, singles, order):
+    """One table whose row i is looked up runs[i] times, one lookup per bag, then `singles` rows once each."""
+    counts = np.concatenate([np.asarray(runs, dtype=np.int64), np.ones(singles, dtype=np.int64)])
+    rows = counts.size
+    indices = np.repeat(np.arange(rows, dtype=np.int64), counts)
+    if order == "mixed":
+        indices = rng.permutation(indices)
+    B = indices.size
+    W, wo, Do = helpers.float_tables(rng, [rows], [D], wdtype, -0.5, 0.5)
+    offsets = np.arange(B + 1, dtype=np.int64)
+    # gradients in steps of 1/64: a run's sum is exact in fp32 whatever the order of its pieces
+    grad = rng.integers(-8, 9, size=(B, D)).astype(np.float32) / 64
+    hs = np.array([0, rows], dtype=np.int64)
+    return 1, W, wo, Do, offsets, indices, None, grad, hs, (rng.random(rows) * 0.1).astype(np.float32), B
+
+
+@pytest.mark.parametrize("D", [4, 32, 64, 128, 256, 512])
+@pytest.mark.parametrize("runs", [
+    [31, 32, 33, 1, 63, 64, 65],                                  # spans of 32: runs that just fit, just do not
+    [16 * 32, 16 * 32 + 1, 23 * 32 + 1, 24 * 32, 25 * 32 + 7],    # either side of what one warp adds alone
+    [40, 5000, 3, 9000],                                          # shared runs in two CTAs
+    [20000],                                                      # the table is one run
+    [4096, 4096, 1, 4095, 4097],                                  # runs that end with a tile, one past it
+], ids=["span", "pieces", "shared", "one", "tile"])
+def test_backward_runs_at_the_edges_of_spans_and_of_the_finish(runs, D):
+    rng = workloads.rng_for(480 + D)
+    *case, B = _runs_case(rng, runs, D, np.float32, 37, "mixed")
+    _check(*case, B, np.float32, np.float32, oracle.SUM, oracle.ROWWISE_ADAGRAD, update_rtol=1e-4)
+
+
+@pytest.mark.parametrize("n,D", [(600_000, 128), (1_300_000, 128), (2_500_000, 128), (700_000, 64)])
+def test_backward_spans_of_every_length(n, D):
+    """The span length follows the number of lookups (64, 128 and 256 positions here, 32 in small batches)."""
+    rng = workloads.rng_for(481)
+    *case, B = _runs_case(rng, [n // 3, 70_000, 257, 4096], D, np.float16, n // 8, "sorted")
+    _check(*case, B, np.float16, np.float32, oracle.SUM, oracle.ROWWISE_ADAGRAD, lr=0.01)
+
+
+@pytest.mark.parametrize("n", [1, 2, 33, 511, 4095, 4096, 4097, 65535, 65536, 65537])
+@pytest.mark.parametrize("T,rows,idx_dtype,weighted", [
+    (1, 7, np.int64, False), (1, 70_001, np.int32, True), (5, 300, np.int32, False), (40, 1000, np.int64, True),
+])
+def test_backward_small_batches_and_the_first_general_one(n, T, rows, idx_dtype, weighted):
+    """Up to 65 536 lookups one launch plans, linearises and sorts; 65 537 take the general path. Tables without
+    a lookup, a table that has nearly all of them, bags that start inside and end with a table."""
+    rng = workloads.rng_for(482 + n + T)
+    share = rng.random(T) ** 8
+    if T > 1:
+        share[rng.integers(T)] = 0.0
+    table = np.sort(rng.choice(T, size=n, p=share / share.sum()))
+    B = 64 if n < 5000 else 600
+    lengths = np.concatenate([rng.multinomial(np.sum(table == t), np.ones(B) / B) for t in range(T)]).astype(np.int64)
+    offsets = np.zeros(T * B + 1, dtype=np.int64)
+    np.cumsum(lengths, out=offsets[1:])
+    indices = rng.integers(0, rows, size=n, dtype=np.int64)
+    indices[rng.random(n) < 0.3] = rows // 2
+    Ds = [16 if t % 2 else 8 for t in range(T)]
+    W, wo, Do = helpers.float_tables(rng, [rows] * T, Ds, np.float32, -0.5, 0.5)
+    hs = np.arange(T + 1, dtype=np.int64) * rows
+    grad = rng.integers(-8, 9, size=(B, int(Do[-1]))).astype(np.float32) / 64
+    psw = rng.random(n).astype(np.float32) if weighted else None
+    mom = (rng.random(T * rows) * 0.1).astype(np.float32)
+    # a row of tens of thousands of weighted lookups: the oracle's own sum is in another order
+    _check(T, W, wo, Do, offsets, indices, psw, grad, hs, mom, B, np.float32, np.float32, oracle.SUM,
+           oracle.ROWWISE_ADAGRAD, idx_dtype=idx_dtype, update_rtol=1e-2 if weighted else 1e-4)
+
+
+@pytest.mark.parametrize("B", [4096, 4097, 20_000])
+def test_backward_small_batch_with_many_bags(B):
+    """Bag starts are kept in shared memory up to 4096 bags per table and searched in place beyond."""
+    rng = workloads.rng_for(483)
+    rows, Ds = [900, 50], [8, 64]
+    case = _backward_case(rng, rows, Ds, B, 0, 2, np.float32, np.float32, oracle.MEAN, oracle.SGD, False)
+    assert case[5].size <= 65536
+    _check(*case, B, np.float32, np.float32, oracle.MEAN, oracle.SGD)
+
+
+def test_backward_small_batch_of_wide_keys():
+    """Row ids of 25 bits: four passes."""
+    rng = workloads.rng_for(484)
+    rows, B = (1 << 24) + 5, 700
+    W, wo, Do = np.zeros(rows * 4, dtype=np.float16), np.zeros(1, dtype=np.int64), np.array([0, 4], dtype=np.int32)
+    offsets = np.arange(B + 1, dtype=np.int64) * 3
+    indices = np.concatenate([rng.integers(0, rows, size=3 * B - 300), np.full(300, rows - 1)]).astype(np.int64)
+    grad = rng.integers(-8, 9, size=(B, 4)).astype(np.float32) / 64
+    hs = np.array([0, rows], dtype=np.int64)
+    _check(1, W, wo, Do, offsets, indices, None, grad, hs, np.zeros(rows, dtype=np.float32), B, np.float16, np.float32,
+           oracle.SUM, oracle.SGD)

@@ -7,7 +7,7 @@
 //               in use); the table is implied by the position
 //   sort        radix_sort.cu, segmented: every table's range is sorted by row on its own, over the
 //               bits of the largest table only (22 bits for 4 M rows, whatever the number of tables)
-//   sweep       groups of lanes walk spans of 256 sorted lookups, summing gradient slices in
+//   sweep       groups of lanes walk spans of 32 to 256 sorted lookups, summing gradient slices in
 //               registers and updating a row where its run of equal keys ends; since the sorted order
 //               is (table, row), only one table's B x D_t slice of the gradient matrix is live in L2
 //   finish      runs that cross span boundaries: their per-span partial sums are added in span order
@@ -79,7 +79,8 @@ struct BwdDev {
   const uint32_t* seg_tile_base;   // [T + 1] first tile of each table
   const uint32_t* total_tiles;     // tiles in use
   const uint4* tile_desc;          // [max_tiles] {begin, count, table, first tile of the table}
-  uint32_t* span_flags;            // [max_tiles * 16]
+  uint32_t* span_flags;            // [max_tiles * spans per tile]
+  int32_t span;                    // sorted positions per span
 };
 
 // ---- linearize -----------------------------------------------------------------------------
@@ -771,7 +772,29 @@ struct ScratchLayout {
   int key_bytes;
   bool sweep;
   int64_t max_long, max_chunks, max_tiles;
+  int span;
 };
+
+// Lanes per row x quads per lane of the sweep: rows of up to 128 elements get one quad per lane of the
+// smallest group that holds them, wider rows the whole warp with several quads per lane.
+constexpr int sweep_group_lanes(int max_D) { return max_D <= 32 ? 8 : (max_D <= 64 ? 16 : 32); }
+
+// Positions per span: the longest that still gives every SM two waves of 32 warps. A warp walks its spans'
+// positions one after the other, so a small batch cut into spans of 256 leaves most of the GPU idle and
+// lasts as long as one span does, and one of a wave and a half waits for the second. Sweep and finish of
+// 11 000 lookups, D = 64: 99 / 57 / 34 / 22 us in spans of 256 / 128 / 64 / 32; of 630 000, D <= 256:
+// 148 / 122 / 122 / 128. With the GPU full anyway, shorter spans only add partial sums (6.9 M lookups:
+// 455 / 454 / 502 / 609 us; 26.7 M: 1270 / 1304 / 1467 / 1850). The partial sums of short spans may take
+// 32 MiB of scratch.
+int span_for(int64_t n, int max_D, int64_t max_tiles) {
+  const int64_t spans_per_warp = 32 / sweep_group_lanes(max_D);   // spans a warp walks side by side
+  const int64_t partial_bytes = int64_t{2} * 4 * (max_D > 0 ? max_D : 1);
+  int span = kMaxSpan;
+  while (span > kMinSpan && n / (span * spans_per_warp) < int64_t{2} * kNumSMs * 32 &&
+         max_tiles * (kSortPlanTile / (span / 2)) * partial_bytes <= (int64_t{32} << 20))
+    span /= 2;
+  return span;
+}
 
 ScratchLayout layout_for(int64_t n, int bits, int max_D, int T) {
   ScratchLayout L{};
@@ -794,9 +817,11 @@ ScratchLayout layout_for(int64_t n, int bits, int max_D, int T) {
   if (L.sweep) {
     // every table's last tile may be partial
     L.max_tiles = sort_plan_max_tiles(n, T);
+    L.span = span_for(n, max_D, L.max_tiles);
+    const size_t spans = static_cast<size_t>(L.max_tiles) * (kSortPlanTile / L.span);
     L.plan = take(sort_plan_bytes(n, T));
-    L.span_flags = take(static_cast<size_t>(L.max_tiles) * kSpansPerTile * 4);
-    L.partials = take(static_cast<size_t>(L.max_tiles) * kSpansPerTile * 2 * row);
+    L.span_flags = take(spans * 4);
+    L.partials = take(spans * 2 * row);
     L.sort = take(radix_sort_planned_scratch_bytes(L.max_tiles));
   } else {
     L.max_long = n / kLongRun + 1;
@@ -890,19 +915,19 @@ int run_backward_wide(BwdDev d, const b200tbe_backward_params* p, const ScratchL
 template <typename WT, typename GT, bool kScaled, int GS, int kC>
 int launch_sweep(const BwdDev& d, int max_tiles, cudaStream_t stream) {
   constexpr int kSpansPerCta = kSweepWarps * (32 / GS);
-  const int64_t ctas = static_cast<int64_t>(max_tiles) * (kSpansPerTile / kSpansPerCta);
+  const int64_t spans = static_cast<int64_t>(max_tiles) * (kSortPlanTile / d.span);
+  const int64_t ctas = spans / kSpansPerCta;
   if (ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
   sweep_runs_kernel<WT, GT, kScaled, GS, kC, sweep_ctas_per_sm<WT, GT, kC>()>
       <<<static_cast<unsigned>(ctas), kSweepThreads, 0, stream>>>(d);
   finish_open_runs_kernel<WT, GS, kC>
-      <<<static_cast<unsigned>(max_tiles), kSpansPerTile * 32, 0, stream>>>(d);
+      <<<static_cast<unsigned>(spans / kFinishSpans), kFinishSpans * 32, 0, stream>>>(d);
   return launch_status();
 }
 
 template <typename WT, typename GT, bool kScaled>
 int dispatch_sweep_shape(const BwdDev& d, int max_tiles, cudaStream_t stream) {
-  // lanes per row x quads per lane: rows of up to 128 elements get one quad per lane of the
-  // smallest group that holds them, wider rows the whole warp with several quads per lane
+  static_assert(sweep_group_lanes(32) == 8 && sweep_group_lanes(64) == 16 && sweep_group_lanes(128) == 32, "");
   if (d.max_D <= 32) return launch_sweep<WT, GT, kScaled, 8, 1>(d, max_tiles, stream);
   if (d.max_D <= 64) return launch_sweep<WT, GT, kScaled, 16, 1>(d, max_tiles, stream);
   if (d.max_D <= 128) return launch_sweep<WT, GT, kScaled, 32, 1>(d, max_tiles, stream);
@@ -967,6 +992,7 @@ int run_backward_sweep(BwdDev d, const b200tbe_backward_params* p, const Scratch
   d.total_tiles = plan.total_tiles;
   d.tile_desc = plan.tile_desc;
   d.span_flags = reinterpret_cast<uint32_t*>(scratch + L.span_flags);
+  d.span = L.span;
 
   // everything above needed only the indices; the gradients are read from here on
   if (p->grad_ready_event != nullptr &&

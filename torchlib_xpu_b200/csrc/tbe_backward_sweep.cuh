@@ -4,8 +4,8 @@
 // seg_start[t+1]) ordered by row, and equal rows are adjacent (a "run"). The reduction is organised
 // by LOOKUP, not by run, because a recommender id stream mixes millions of one-lookup runs with
 // runs of a hundred thousand lookups:
-//   * every tile of the sort plan (4096 sorted positions of one table) is cut into 16 spans of 256
-//     positions; a group of GS lanes sweeps one span from left to right, each lane holding kC quads
+//   * every tile of the sort plan (4096 sorted positions of one table) is cut into spans of 256
+//     positions (fewer in small batches); a group of GS lanes sweeps one span from left to right, each lane holding kC quads
 //     of 4 elements of the running sum (quad c of lane l = elements (c * GS + l) * 4 ...), so one
 //     load instruction of a group reads contiguous bytes of one gradient slice. A warp carries
 //     32 / GS groups, i.e. that many consecutive spans, through one instruction stream;
@@ -27,8 +27,12 @@
 // Part of tbe_backward.cu: included there inside its namespace, after BwdDev and bag_length.
 #pragma once
 
-constexpr int kSpan = 256;                                  // sorted positions per span
-constexpr int kSpansPerTile = kSortPlanTile / kSpan;        // 16
+// Sorted positions per span (BwdDev::span, a power of two): 256 where the spans fill the GPU several
+// times over, fewer where they would not (span_for in tbe_backward.cu).
+constexpr int kMaxSpan = 256;
+constexpr int kMinSpan = 32;                                 // at least the widest group's batch
+// spans per CTA of the finish kernel; a tile's spans are a whole number of such groups
+constexpr int kFinishSpans = kSortPlanTile / kMaxSpan;       // 16
 // One warp per CTA: spans finish at very different times (a span inside a long run is pure
 // streaming, a span of one-lookup runs updates a row every other position), and a CTA keeps its
 // slot until its slowest warp is done. Measured on the bench step: 4 warps per CTA 9.65 ms for the
@@ -563,25 +567,27 @@ __global__ void __launch_bounds__(kSweepThreads, kMinCtas)
     sweep_runs_kernel(const __grid_constant__ BwdDev p) {
   constexpr int NG = 32 / GS;
   constexpr int kSpansPerCta = kSweepWarps * NG;
-  static_assert(kSpansPerTile % kSpansPerCta == 0, "a CTA's spans lie in one tile");
-  constexpr int kCtasPerTile = kSpansPerTile / kSpansPerCta;
+  static_assert(kFinishSpans % kSpansPerCta == 0, "a CTA's spans lie in one tile");
+  const int span = p.span;
+  const uint32_t spans_per_tile = kSortPlanTile / span;
+  const uint32_t ctas_per_tile = spans_per_tile / kSpansPerCta;
 
-  const uint32_t tile = blockIdx.x / kCtasPerTile;
+  const uint32_t tile = blockIdx.x / ctas_per_tile;
   if (tile >= __ldg(p.total_tiles)) return;
   const uint4 td = __ldg(p.tile_desc + tile);   // {begin, count, table, first tile of the table}
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   SpanCtx sc;
   sc.grp = lane / GS;
   sc.gl = lane % GS;
-  const int warp_span0 = static_cast<int>(blockIdx.x % kCtasPerTile) * kSpansPerCta + warp * NG;
+  const int warp_span0 = static_cast<int>(blockIdx.x - tile * ctas_per_tile) * kSpansPerCta + warp * NG;
   const int tile_n = static_cast<int>(td.y);
-  if (warp_span0 * kSpan >= tile_n) return;
+  if (warp_span0 * span >= tile_n) return;
   const int span_in_tile = warp_span0 + sc.grp;
-  sc.span_id = tile * kSpansPerTile + span_in_tile;
+  sc.span_id = tile * spans_per_tile + span_in_tile;
   const int t = static_cast<int>(td.z);
-  const int s_off = span_in_tile * kSpan;
-  sc.s_count = s_off >= tile_n ? 0 : (tile_n - s_off < kSpan ? tile_n - s_off : kSpan);
-  sc.cnt0 = tile_n - warp_span0 * kSpan < kSpan ? tile_n - warp_span0 * kSpan : kSpan;
+  const int s_off = span_in_tile * span;
+  sc.s_count = s_off >= tile_n ? 0 : (tile_n - s_off < span ? tile_n - s_off : span);
+  sc.cnt0 = tile_n - warp_span0 * span < span ? tile_n - warp_span0 * span : span;
   sc.s_begin = td.x + s_off;
   sc.seg_begin = __ldg(p.seg_start + t);
   sc.seg_end = __ldg(p.seg_start + t + 1);
@@ -599,44 +605,47 @@ __global__ void __launch_bounds__(kSweepThreads, kMinCtas)
   }
 }
 
-// One CTA per tile, one warp per span: a span whose last run continues to the right owns that run. Its
-// warp adds the run's pieces in span order -- the span's tail slot, then the head slot of every
-// following span up to and including the first one that the run does not pass through -- and updates
-// the row. Group g takes pieces g, g + NG, ...
+// One CTA per 16 consecutive spans of a tile, one warp per span: a span whose last run continues to the
+// right owns that run. Its warp adds the run's pieces in span order -- the span's tail slot, then the
+// head slot of every following span up to and including the first one that the run does not pass
+// through -- and updates the row. Group g takes pieces g, g + NG, ...
 // A run of more than kAlonePieces pieces (a hot row: 150 000 lookups leave almost 600) would be a chain
 // of memory round trips for one warp, 0.2 ms whatever the rest of the launch does. It reaches past the
-// tile's end, so a tile owns at most one: the tile's sixteen warps share it, each adding a contiguous
+// CTA's spans, so a CTA owns at most one: its sixteen warps share it, each adding a contiguous
 // sixteenth of the pieces, and the first warp adds the sixteen sums in order. (16 tables x 4 M rows,
 // B 65536, Zipf ids, 26.7 M lookups: the training step 2.68 -> 2.56 ms; 26 tables x 1 M rows, B 8192:
 // 0.898 -> 0.877 ms.)
 constexpr int kAlonePieces = 24;
-static_assert(kAlonePieces >= kSpansPerTile, "a run that is shared reaches past its tile's end");
+static_assert(kAlonePieces >= kFinishSpans, "a run that is shared reaches past its CTA's spans");
 
 template <typename WT, int GS, int kC>
-__global__ void __launch_bounds__(kSpansPerTile * 32)
+__global__ void __launch_bounds__(kFinishSpans * 32)
     finish_open_runs_kernel(const __grid_constant__ BwdDev p) {
   constexpr int NG = 32 / GS;
   constexpr int quad_w = GS * 4 * static_cast<int>(sizeof(WT));
-  __shared__ float4 shared_sum[kSpansPerTile][GS * kC];
-  __shared__ uint32_t shared_span, shared_heads;   // the tile's shared run; heads 0: none
+  __shared__ float4 shared_sum[kFinishSpans][GS * kC];
+  __shared__ uint32_t shared_span, shared_heads;   // the CTA's shared run; heads 0: none
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane / GS, gl = lane % GS;
-  const uint32_t tile = blockIdx.x;
+  const int span = p.span;
+  const uint32_t spans_per_tile = kSortPlanTile / span;
+  const uint32_t span0 = blockIdx.x * kFinishSpans;   // all of the CTA's spans lie in one tile
+  const uint32_t tile = span0 / spans_per_tile;
   const uint32_t live_tiles = __ldg(p.total_tiles);
   if (tile >= live_tiles) return;
   const uint4 td = __ldg(p.tile_desc + tile);
   const int tile_n = static_cast<int>(td.y);
   const int t = static_cast<int>(td.z);
-  const uint32_t my_span = tile * kSpansPerTile + warp;
+  const uint32_t my_span = span0 + warp;
   if (threadIdx.x == 0) shared_heads = 0;
   __syncthreads();
 
   // pieces after the tail slot: one per following span, the last being the first span that is not
   // passed through (flags of spans the run cannot reach are never decisive)
-  const bool owner = warp * kSpan < tile_n && (p.span_flags[my_span] & kSpanTailOwner) != 0;
+  const bool owner = static_cast<int>((my_span - tile * spans_per_tile) * span) < tile_n && (p.span_flags[my_span] & kSpanTailOwner) != 0;
   uint32_t heads = 0;
   if (owner) {
-    const uint32_t span_limit = live_tiles * kSpansPerTile;
+    const uint32_t span_limit = live_tiles * spans_per_tile;
     constexpr int kAhead = 4;   // 128 flags per step
     for (uint32_t v = my_span + 1;; v += 32 * kAhead) {
       uint32_t stop[kAhead];
@@ -671,10 +680,10 @@ __global__ void __launch_bounds__(kSpansPerTile * 32)
 #pragma unroll
   for (int c = 0; c < kC; ++c) on[c] = (c * GS + gl) * 4 < D;
 
-  // acc = pieces [first, last) of the run that `span` owns: piece 0 = its tail slot, piece i >= 1 = the
-  // head slot of span + i. Eight pieces are requested before the first is added.
+  // acc = pieces [first, last) of the run that `owner_span` owns: piece 0 = its tail slot, piece i >= 1 =
+  // the head slot of owner_span + i. Eight pieces are requested before the first is added.
   const float* lane_base = p.partials + gl * 4;
-  auto sum_pieces = [&](uint32_t span, uint32_t first, uint32_t last) {
+  auto sum_pieces = [&](uint32_t owner_span, uint32_t first, uint32_t last) {
     constexpr int kPieces = 8 / kC;
 #pragma unroll
     for (int c = 0; c < kC; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -684,7 +693,7 @@ __global__ void __launch_bounds__(kSpansPerTile * 32)
       for (int u = 0; u < kPieces; ++u) {
         const uint32_t i = i0 + u * NG;
         const uint32_t j = i < last ? i : i0;
-        const int64_t slot = j == 0 ? 2 * static_cast<int64_t>(span) + 1 : 2 * static_cast<int64_t>(span + j);
+        const int64_t slot = j == 0 ? 2 * static_cast<int64_t>(owner_span) + 1 : 2 * static_cast<int64_t>(owner_span + j);
         const float* src = lane_base + slot * p.max_D;
 #pragma unroll
         for (int c = 0; c < kC; ++c) {
@@ -714,14 +723,14 @@ __global__ void __launch_bounds__(kSpansPerTile * 32)
       }
     }
   };
-  // updates the row of the run that `span` owns with the gradient in acc
-  auto update_row = [&](uint32_t span) {
+  // updates the row of the run that `owner_span` owns with the gradient in acc
+  auto update_row = [&](uint32_t owner_span) {
     float sq = sum_squares<kC>(acc);
 #pragma unroll
     for (int o = GS >> 1; o > 0; o >>= 1) sq += __shfl_xor_sync(kFullMask, sq, o);
     if (sq == 0.f) return;
-    const int s_off = static_cast<int>(span % kSpansPerTile) * kSpan;
-    const int s_count = tile_n - s_off < kSpan ? tile_n - s_off : kSpan;
+    const int s_off = static_cast<int>(owner_span - tile * spans_per_tile) * span;
+    const int s_count = tile_n - s_off < span ? tile_n - s_off : span;
     const uint32_t row = __ldg(reinterpret_cast<const uint32_t*>(p.sorted_keys) + td.x + s_off + s_count - 1);
     char* wrow = p.dev_weights +
                  (__ldg(p.weights_offsets + t) + static_cast<int64_t>(row) * D) * static_cast<int64_t>(sizeof(WT)) +
@@ -749,7 +758,7 @@ __global__ void __launch_bounds__(kSpansPerTile * 32)
   __syncthreads();
   const uint32_t pieces = shared_heads + 1;
   if (pieces == 1) return;
-  const uint32_t each = (pieces + kSpansPerTile - 1) / kSpansPerTile;
+  const uint32_t each = (pieces + kFinishSpans - 1) / kFinishSpans;
   const uint32_t first = warp * each < pieces ? warp * each : pieces;
   sum_pieces(shared_span, first, first + each < pieces ? first + each : pieces);
 #pragma unroll
@@ -761,7 +770,7 @@ __global__ void __launch_bounds__(kSpansPerTile * 32)
   for (int c = 0; c < kC; ++c) {
     acc[c] = shared_sum[0][c * GS + gl];
 #pragma unroll
-    for (int w = 1; w < kSpansPerTile; ++w) {
+    for (int w = 1; w < kFinishSpans; ++w) {
       const float4 x = shared_sum[w][c * GS + gl];
       acc[c].x += x.x;
       acc[c].y += x.y;
