@@ -329,6 +329,30 @@ B200TBE_API int b200tbe_permute_segments(const void* in, void* out, const void* 
                                          b200tbe_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------------
+ * torch.ops.fbgemm.permute_2D_sparse_data in two calls. lengths is [rows][cols] (elements of
+ * length_bytes, 4 or 8), the values hold the rows' elements one row after the other; row j of the
+ * result is row perm[j].
+ * b200tbe_permute_row_starts writes in_start[out_rows] (where output row j's elements begin in the
+ * input), out_offsets[out_rows + 1] (where they begin in the output) and, when permuted_lengths is
+ * not null, the permuted [out_rows][cols] lengths. A perm entry outside [0, rows) fails a device
+ * assertion.
+ * b200tbe_permute_rows moves one array of elem_bytes-wide elements (2, 4 or 8) and, when in2 is not
+ * null, a second one of elem2_bytes (ids and their per-sample weights: one launch for 8- or 4-byte
+ * elements with 4-byte ones). Output elements past out_offsets[out_rows] are left as they are.
+ * ---------------------------------------------------------------------------------------------- */
+B200TBE_API size_t b200tbe_permute_row_starts_scratch_bytes(int64_t rows, int64_t cols);
+B200TBE_API int b200tbe_permute_row_starts(const void* lengths, const void* perm, void* permuted_lengths,
+                                           int64_t* in_start, int64_t* out_offsets, int64_t rows,
+                                           int64_t cols, int64_t out_rows, int32_t length_bytes,
+                                           int32_t perm_bytes, void* scratch, size_t scratch_bytes,
+                                           b200tbe_stream_t stream);
+B200TBE_API int b200tbe_permute_rows(const void* in, void* out, int32_t elem_bytes, const void* in2,
+                                     void* out2, int32_t elem2_bytes, const int64_t* in_start,
+                                     const int64_t* out_offsets, int64_t out_rows, int64_t total_elems,
+                                     b200tbe_stream_t stream);
+
+
+/* ------------------------------------------------------------------------------------------------
  * Jagged tensors. values is [total_rows, inner_size]; dense is [outer_size, max_lengths[0], ...,
  * max_lengths[n-1], inner_size]; offsets[d] is the d-th level's offsets array (offsets[0] has
  * outer_size + 1 entries). Elements are moved as raw bytes, so any dtype of elem_bytes 1, 2, 4 or 8

@@ -201,3 +201,31 @@ def test_permute_2d_sparse_data_rows_may_repeat_or_drop():
                                                              dev(indices.astype(np.int32)), None, int(want_idx.size))
     assert none is None and np.array_equal(pi2.cpu().numpy(), want_idx.astype(np.int32))
     assert np.array_equal(pl2.cpu().numpy(), lengths[permute].astype(np.int32))
+
+
+@pytest.mark.parametrize("T,B,hi,P", [(1, 1, 5, 1), (3, 4096, 3, 3), (3, 4097, 9, 7), (255, 33, 40, 256), (257, 8, 400, 257),
+                                      (1500, 5, 3, 1300), (7, 0, 1, 7), (40, 3, 0, 40)])
+@pytest.mark.parametrize("id_dtype,w_dtype,len_dtype,perm_dtype", [
+    (torch.int64, torch.float32, torch.int32, torch.int32), (torch.int32, torch.float32, torch.int64, torch.int64),
+    (torch.int64, torch.float64, torch.int16, torch.int32), (torch.int32, torch.float16, torch.int32, torch.int64),
+    (torch.int64, None, torch.int64, torch.int32),
+])
+def test_permute_2d_sparse_data_shapes_and_types(T, B, hi, P, id_dtype, w_dtype, len_dtype, perm_dtype):
+    """Rows that are empty, shorter and far longer than a tile, more rows than one search round holds, rows that
+    repeat or are left out; every route of element, length and permutation types. Bytes move: exact."""
+    rng = workloads.rng_for(1410 + T)
+    lengths = torch.from_numpy(rng.integers(0, hi + 1, size=(T, B))).to(len_dtype)
+    if T > 4 and B:
+        lengths[1:3] = 0
+    total = int(lengths.sum())
+    indices = torch.from_numpy(rng.integers(0, 1 << 31, size=total)).to(id_dtype)
+    weights = None if w_dtype is None else torch.from_numpy(rng.standard_normal(total)).to(w_dtype)
+    permute = torch.from_numpy(rng.permutation(T) if P == T else rng.integers(0, T, size=P)).to(perm_dtype)
+    rows = lengths.long().sum(1)
+    start = torch.cumsum(rows, 0) - rows
+    at = torch.cat([torch.arange(int(start[t]), int(start[t] + rows[t])) for t in permute.tolist()] + [torch.empty(0, dtype=torch.long)])
+    cuda = lambda x: None if x is None else x.cuda()  # noqa: E731
+    for given in (None, at.numel()):
+        pl, pi, pw = torch.ops.fbgemm.permute_2D_sparse_data(cuda(permute), cuda(lengths), cuda(indices), cuda(weights), given)
+        assert torch.equal(pl.cpu(), lengths[permute.long()]) and torch.equal(pi.cpu(), indices[at])
+        assert pw is None if weights is None else torch.equal(pw.cpu(), weights[at])

@@ -91,7 +91,9 @@ EXPORTS = (
     "b200tbe_backward_scratch_bytes", "b200tbe_backward", "b200tbe_radix_sort_scratch_bytes",
     "b200tbe_radix_sort_pairs", "b200tbe_radix_sort_segments_scratch_bytes",
     "b200tbe_radix_sort_segments", "b200tbe_radix_sort_pairs_static_max",
-    "b200tbe_radix_sort_pairs_static", "b200tbe_exchange_push", "b200tbe_permute_segments", "b200tbe_quantized_row_bytes",
+    "b200tbe_radix_sort_pairs_static", "b200tbe_exchange_push", "b200tbe_permute_segments",
+    "b200tbe_permute_row_starts_scratch_bytes", "b200tbe_permute_row_starts", "b200tbe_permute_rows",
+    "b200tbe_quantized_row_bytes",
     "b200tbe_quantize_rows", "b200tbe_dequantize_rows", "b200tbe_nv12_to_rgb", "b200tbe_jagged_to_padded_dense", "b200tbe_dense_to_jagged",
     "b200tbe_jagged_dense_elementwise_add",
 )

@@ -349,7 +349,7 @@ Tensor jagged_2d_to_dense_autograd(const Tensor& values, const Tensor& offsets, 
 // ---- permute_2D_sparse_data -----------------------------------------------------------------------
 // lengths is [T, B], indices (and weights) hold the T rows' ids one row after the other; row j of
 // the result is row permute[j] of the input (rows may repeat or be left out, so the result can be
-// longer or shorter than the input). Whole rows move as segments of b200tbe_permute_segments.
+// longer or shorter than the input): two kernels find the rows' places, one moves ids and weights.
 std::tuple<Tensor, Tensor, c10::optional<Tensor>> permute_2d_sparse_data(
     const Tensor& permute, const Tensor& lengths, const Tensor& indices,
     const c10::optional<Tensor>& weights, c10::optional<int64_t> permuted_lengths_sum) {
@@ -359,39 +359,56 @@ std::tuple<Tensor, Tensor, c10::optional<Tensor>> permute_2d_sparse_data(
   TORCH_CHECK(lengths.dim() == 2, "lengths must be [T, B]");
   TORCH_CHECK(permute.scalar_type() == at::kInt || permute.scalar_type() == at::kLong,
               "permute must be int32 or int64");
+  TORCH_CHECK(permute.dim() <= 1, "permute must be a vector");
+  TORCH_CHECK(permute.device() == lengths.device() && lengths.device() == indices.device(),
+              "permute, lengths and indices must be on the same device");
+  const int64_t T = lengths.size(0), B = lengths.size(1), P = permute.numel();
+  TORCH_CHECK(T > 0 || P == 0, "permute selects rows of an empty matrix");
+  const bool weighted = weights.has_value() && weights->defined();
+  auto check_element = [](const Tensor& t, const char* what) {
+    const int64_t eb = static_cast<int64_t>(t.element_size());
+    TORCH_CHECK(eb == 2 || eb == 4 || eb == 8, what, ": elements of 2, 4 or 8 bytes");
+  };
+  check_element(indices, "indices");
+  if (weighted) {
+    check_cuda_contig(*weights, "weights");
+    TORCH_CHECK(weights->numel() == indices.numel(), "weights and indices differ in length");
+    check_element(*weights, "weights");
+  }
   c10::cuda::CUDAGuard guard(indices.device());
-  const Tensor permuted_lengths = lengths.index_select(0, permute);
-  const Tensor row_len = lengths.to(at::kLong).sum(1);
-  Tensor in_off = at::zeros({row_len.numel() + 1}, row_len.options());
-  in_off.slice(0, 1).copy_(row_len.cumsum(0));
-  const Tensor out_len = row_len.index_select(0, permute);
-  Tensor out_off = at::zeros({out_len.numel() + 1}, out_len.options());
-  out_off.slice(0, 1).copy_(out_len.cumsum(0));
+  // lengths of another type are summed as int64 and gathered as what they are
+  const bool plain = lengths.scalar_type() == at::kInt || lengths.scalar_type() == at::kLong;
+  const Tensor len = plain ? lengths : lengths.to(at::kLong);
+  const Tensor permuted_lengths = plain ? at::empty({P, B}, lengths.options()) : lengths.index_select(0, permute);
+  const size_t scratch_bytes = b200tbe_permute_row_starts_scratch_bytes(T, B);
+  // [0, P): where the output rows' elements begin in the input; [P, 2P]: in the output; then scratch
+  const Tensor words =
+      at::empty({2 * P + 1 + static_cast<int64_t>(scratch_bytes / 8)}, lengths.options().dtype(at::kLong));
+  int64_t* in_start = words.data_ptr<int64_t>();
+  int64_t* out_offsets = in_start + P;
+  check_status(b200tbe_permute_row_starts(len.data_ptr(), permute.data_ptr(),
+                                          plain ? permuted_lengths.data_ptr() : nullptr, in_start, out_offsets, T, B,
+                                          P, static_cast<int32_t>(len.element_size()),
+                                          static_cast<int32_t>(permute.element_size()), out_offsets + P + 1,
+                                          scratch_bytes, current_stream()),
+               "permute_2D_sparse_data");
   int64_t total = 0;
   if (permuted_lengths_sum.has_value()) {
     total = *permuted_lengths_sum;
   } else {
-    total = out_off[-1].item<int64_t>();  // one synchronising read, as in fbgemm_gpu
+    total = words[2 * P].item<int64_t>();  // one synchronising read, as in fbgemm_gpu
   }
   TORCH_CHECK(total >= 0, "permuted_lengths_sum must be non-negative");
-  auto move = [&](const Tensor& src, const char* what) {
-    Tensor dst = at::empty({total}, src.options());
-    const int64_t eb = static_cast<int64_t>(src.element_size());
-    TORCH_CHECK(eb == 2 || eb == 4 || eb == 8, what, ": elements of 2, 4 or 8 bytes");
-    check_status(b200tbe_permute_segments(src.data_ptr(), dst.data_ptr(), in_off.data_ptr(),
-                                          out_off.data_ptr(), permute.data_ptr(), permute.numel(),
-                                          total, static_cast<int32_t>(eb), 8,
-                                          static_cast<int32_t>(permute.element_size()), current_stream()),
-                 "permute_2D_sparse_data");
-    return dst;
-  };
-  Tensor permuted_indices = move(indices, "indices");
+  Tensor permuted_indices = at::empty({total}, indices.options());
   c10::optional<Tensor> permuted_weights;
-  if (weights.has_value() && weights->defined()) {
-    check_cuda_contig(*weights, "weights");
-    TORCH_CHECK(weights->numel() == indices.numel(), "weights and indices differ in length");
-    permuted_weights = move(*weights, "weights");
-  }
+  if (weighted) permuted_weights = at::empty({total}, weights->options());
+  check_status(b200tbe_permute_rows(indices.data_ptr(), permuted_indices.data_ptr(),
+                                    static_cast<int32_t>(indices.element_size()),
+                                    weighted ? weights->data_ptr() : nullptr,
+                                    weighted ? permuted_weights->data_ptr() : nullptr,
+                                    weighted ? static_cast<int32_t>(weights->element_size()) : 0, in_start,
+                                    out_offsets, P, total, current_stream()),
+               "permute_2D_sparse_data");
   return {permuted_lengths, permuted_indices, permuted_weights};
 }
 

@@ -4,11 +4,19 @@
 //
 // Segments range from empty bags to whole tables, so the work is split by output ELEMENT, not by
 // segment: a CTA owns a tile of consecutive output elements, finds the segment of its first element
-// by a CTA-wide 256-ary search over the output offsets, walks the segment boundaries of the tile into shared
-// memory once, marks which of them holds each element of the tile (first elements marked, a running
-// maximum spreads the marks), and then every thread copies elements whose source position is the input
-// start of their segment plus their distance from its output start. Reads and writes are coalesced inside
-// a segment; per element the traffic is its bytes in and out plus one shared-memory lookup.
+// by a CTA-wide 256-ary search over the output offsets (256 segments or fewer: none needed), lists the
+// segments of the tile in shared memory once, each as the distance from its output to its input position,
+// and marks which of them holds each element of the tile (first elements marked, a running maximum spreads
+// the marks). Then every thread copies elements, eight loads in flight. A tile inside one segment -- most
+// tiles, where whole tables move -- needs no map at all. Ids and their per-sample weights go through one
+// launch: the second array costs its bytes only, not another search and map.
+//
+// Bound by memory: 26.7 M ids of 8 bytes and as many 4-byte weights in 128 segments take
+// 108 us (5.9 TB/s); in two launches that built a map for every tile it was 92 + 69 us.
+#include <assert.h>
+
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace b200tbe {
@@ -39,18 +47,31 @@ __device__ __forceinline__ int64_t segment_of(const void* off, int64_t n, int64_
   return lo;
 }
 
-template <typename ElemT, typename OffT, typename PermT>
+struct NoElem {};   // no second array
+
+// Output segment j is input segment perm[j], which starts at in_offsets[perm[j]] (kStarts: in_offsets[j] is
+// already the start of segment j's source, and perm is not read).
+template <typename ElemT, typename Elem2T, typename OffT, typename PermT, bool kStarts>
 __global__ void __launch_bounds__(kPermThreads)
-    permute_segments_kernel(const ElemT* __restrict__ in, ElemT* __restrict__ out,
-                            const void* __restrict__ in_offsets, const void* __restrict__ out_offsets,
-                            const PermT* __restrict__ perm, int64_t num_segments, int64_t total) {
-  __shared__ int64_t seg_out_start[kPermMaxSegs];   // output start of the tile's k-th segment
-  __shared__ int64_t seg_in_start[kPermMaxSegs];    // input start of the same segment
-  __shared__ int seg_count;
+    permute_segments_kernel(const ElemT* __restrict__ in, ElemT* __restrict__ out, const Elem2T* __restrict__ in2,
+                            Elem2T* __restrict__ out2, const void* __restrict__ in_offsets,
+                            const void* __restrict__ out_offsets, const PermT* __restrict__ perm,
+                            int64_t num_segments, int64_t total) {
+  constexpr bool kTwo = !std::is_same<Elem2T, NoElem>::value;
+  // the tile's k-th segment: input position minus output position of its elements
+  __shared__ int64_t seg_delta[kPermMaxSegs];
+  __shared__ __align__(16) uint16_t slot_of[kPermTile];   // listed segment of each element
+  __shared__ int warp_live[kPermThreads / 32];
+  __shared__ int warp_carry[kPermThreads / 32];
   __shared__ int64_t first_seg;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t tile0 = static_cast<int64_t>(blockIdx.x) * kPermTile;
   const int64_t tile1 = tile0 + kPermTile < total ? tile0 + kPermTile : total;
-  {
+  auto source_of = [&](int64_t seg) {
+    return load_off<OffT>(in_offsets, kStarts ? seg : static_cast<int64_t>(perm[seg]));
+  };
+  int64_t s = 0;
+  if (num_segments > kPermThreads) {
     // the segment of the tile's first element, searched by the whole CTA: 256 probes per round
     // narrow the range 256-fold, so 22 bits of segments take 3 dependent loads instead of 22
     int64_t lo = 0, n = num_segments;
@@ -63,88 +84,85 @@ __global__ void __launch_bounds__(kPermThreads)
       n = n - c * step < step ? n - c * step : step;
     }
     if (threadIdx.x == 0) first_seg = lo;
+    __syncthreads();
+    s = first_seg;
   }
-  __syncthreads();
+  {
+    uint4* z = reinterpret_cast<uint4*>(slot_of);
+    for (int q = threadIdx.x; q < kPermTile / 8; q += kPermThreads) z[q] = make_uint4(0u, 0u, 0u, 0u);
+  }
   // the non-empty segments that intersect the tile, in order; threads take candidates round-robin
-  // and a segment's slot is its rank among the non-empty ones, found with a block-wide count
-  int64_t s = first_seg;
+  // and a segment's slot is its rank among the non-empty ones, found with a block-wide count. Every
+  // segment marks its first element with its slot (slots grow with the position).
   int filled = 0;
   bool overflow = false;
   while (true) {
     const int64_t cand = s + threadIdx.x;
-    bool live = false;
+    bool live = false, past = true;
     int64_t o0 = 0;
     if (cand < num_segments) {
       o0 = load_off<OffT>(out_offsets, cand);
       const int64_t o1 = load_off<OffT>(out_offsets, cand + 1);
       live = o0 < tile1 && o1 > o0 && o1 > tile0;
+      past = o1 >= tile1;
     }
-    // rank of this thread's segment among the live ones of this round
     const unsigned ballot = __ballot_sync(kFullMask, live);
-    __shared__ int warp_live[kPermThreads / 32];
-    if ((threadIdx.x & 31) == 0) warp_live[threadIdx.x >> 5] = __popc(ballot);
-    __syncthreads();
+    if (lane == 0) warp_live[warp] = __popc(ballot);
+    // done when the round reached the end of the segments or the tile (also: slot_of is clear)
+    const bool last_round = __syncthreads_or(threadIdx.x == kPermThreads - 1 && past);
     int before = 0, round_total = 0;
     for (int w = 0; w < kPermThreads / 32; ++w) {
-      if (w < static_cast<int>(threadIdx.x >> 5)) before += warp_live[w];
+      if (w < warp) before += warp_live[w];
       round_total += warp_live[w];
     }
-    const int slot = filled + before + __popc(ballot & ((1u << (threadIdx.x & 31)) - 1u));
-    if (live) {
-      if (slot < kPermMaxSegs) {
-        seg_out_start[slot] = o0;
-        seg_in_start[slot] = load_off<OffT>(in_offsets, static_cast<int64_t>(perm[cand]));
-      }
+    const int slot = filled + before + __popc(ballot & ((1u << lane) - 1u));
+    if (live && slot < kPermMaxSegs) {
+      seg_delta[slot] = source_of(cand) - o0;
+      const int64_t at = o0 - tile0;
+      slot_of[at > 0 ? at : 0] = static_cast<uint16_t>(slot);
     }
     filled += round_total;
-    // done when the round reached the end of the segments or a segment that starts past the tile
-    const bool last_round = s + kPermThreads >= num_segments ||
-                            load_off<OffT>(out_offsets, s + kPermThreads) >= tile1;
+    overflow = filled > kPermMaxSegs;
     __syncthreads();
-    if (filled > kPermMaxSegs) overflow = true;
     if (last_round || overflow) break;
     s += kPermThreads;
   }
-  if (threadIdx.x == 0) seg_count = filled < kPermMaxSegs ? filled : kPermMaxSegs;
-  __syncthreads();
-  const int count = seg_count;
-  // Which listed segment holds each element of the tile: every segment marks its first element with
-  // its slot (slots grow with the position), and a running maximum over the tile spreads the marks.
-  // Thread t scans elements [16 t, 16 t + 16); the carry across threads is a warp / CTA max-scan.
-  __shared__ __align__(16) uint16_t slot_of[kPermTile];
-  __shared__ int warp_carry[kPermThreads / 32];
-  if (!overflow) {
-    uint4* z = reinterpret_cast<uint4*>(slot_of);
-    for (int q = threadIdx.x; q < kPermTile / 8; q += kPermThreads) z[q] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    for (int k = threadIdx.x; k < count; k += kPermThreads) {
-      const int64_t at = seg_out_start[k] - tile0;
-      slot_of[at > 0 ? at : 0] = static_cast<uint16_t>(k);
-    }
-    __syncthreads();
-    uint16_t* mine = slot_of + threadIdx.x * kPermItems;
+  // offsets that end before `total` leave the rest of the output as it is
+  const int64_t end = load_off<OffT>(out_offsets, num_segments);
+  const int64_t live1 = tile1 < end ? tile1 : end;
+  if (filled > 1 && !overflow) {
+    // a running maximum over the tile spreads the marks: thread t scans elements [16 t, 16 t + 16); the
+    // carry across threads is a warp / CTA max-scan
+    uint4* mine = reinterpret_cast<uint4*>(slot_of + threadIdx.x * kPermItems);
+    static_assert(kPermItems == 16, "two 16-byte words of marks per thread");
+    uint4 m[2] = {mine[0], mine[1]};
+    uint16_t* e = reinterpret_cast<uint16_t*>(m);
     int run = 0;
 #pragma unroll
-    for (int j = 0; j < kPermItems; ++j) run = max(run, static_cast<int>(mine[j]));
+    for (int j = 0; j < kPermItems; ++j) run = max(run, static_cast<int>(e[j]));
     int incl = run;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int up = __shfl_up_sync(kFullMask, incl, o);
-      if ((threadIdx.x & 31) >= o) incl = max(incl, up);
+      if (lane >= o) incl = max(incl, up);
     }
-    if ((threadIdx.x & 31) == 31) warp_carry[threadIdx.x >> 5] = incl;
+    if (lane == 31) warp_carry[warp] = incl;
     __syncthreads();
     int carry = __shfl_up_sync(kFullMask, incl, 1);
-    if ((threadIdx.x & 31) == 0) carry = 0;
-    for (int w = 0; w < static_cast<int>(threadIdx.x >> 5); ++w) carry = max(carry, warp_carry[w]);
+    if (lane == 0) carry = 0;
+    for (int w = 0; w < warp; ++w) carry = max(carry, warp_carry[w]);
 #pragma unroll
     for (int j = 0; j < kPermItems; ++j) {
-      carry = max(carry, static_cast<int>(mine[j]));
-      mine[j] = static_cast<uint16_t>(carry);
+      carry = max(carry, static_cast<int>(e[j]));
+      e[j] = static_cast<uint16_t>(carry);
     }
+    mine[0] = m[0];
+    mine[1] = m[1];
     __syncthreads();
   }
-  // eight elements at a time: their source positions first, then all eight loads, then the stores
+  const bool one = filled == 1;
+  const int64_t one_delta = seg_delta[0];
+  // eight elements at a time: their source positions first, then all loads, then the stores
   constexpr int kBatch = 8;
 #pragma unroll
   for (int k0 = 0; k0 < kPermItems; k0 += kBatch) {
@@ -154,45 +172,184 @@ __global__ void __launch_bounds__(kPermThreads)
       const int e = (k0 + u) * kPermThreads + threadIdx.x;
       const int64_t i = tile0 + e;
       src[u] = -1;
-      if (i >= tile1) continue;
-      if (!overflow) {
-        const int slot = slot_of[e];
-        src[u] = seg_in_start[slot] + (i - seg_out_start[slot]);
+      if (i >= live1) continue;
+      if (one) {
+        src[u] = i + one_delta;
+      } else if (!overflow) {
+        src[u] = i + seg_delta[slot_of[e]];
       } else {
         // more segment boundaries in one tile than the table holds (thousands of one-element
         // segments): every element searches the global offsets itself
         // (the last segment that starts at or before i is the non-empty one that holds it)
         const int64_t seg = segment_of<OffT>(out_offsets, num_segments, i);
-        src[u] = load_off<OffT>(in_offsets, static_cast<int64_t>(perm[seg])) + (i - load_off<OffT>(out_offsets, seg));
+        src[u] = source_of(seg) + (i - load_off<OffT>(out_offsets, seg));
       }
     }
     ElemT v[kBatch];
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u)
-      if (src[u] >= 0) v[u] = in[src[u]];
+    Elem2T v2[kTwo ? kBatch : 1];
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
+      if (src[u] < 0) continue;
+      v[u] = in[src[u]];
+      if constexpr (kTwo) v2[u] = in2[src[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (src[u] < 0) continue;
       const int64_t i = tile0 + static_cast<int64_t>(k0 + u) * kPermThreads + threadIdx.x;
-      if (src[u] >= 0) out[i] = v[u];
+      out[i] = v[u];
+      if constexpr (kTwo) out2[i] = v2[u];
     }
   }
 }
 
-template <typename ElemT, typename OffT>
-int launch_perm(const void* in, void* out, const void* in_offsets, const void* out_offsets,
-                const void* perm, int perm_bytes, int64_t num_segments, int64_t total,
+template <typename ElemT, typename Elem2T, typename OffT, typename PermT, bool kStarts>
+int launch_perm(const void* in, void* out, const void* in2, void* out2, const void* in_offsets,
+                const void* out_offsets, const void* perm, int64_t num_segments, int64_t total,
                 cudaStream_t stream) {
   const int64_t ctas = (total + kPermTile - 1) / kPermTile;
   if (ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
-  if (perm_bytes == 4) {
-    permute_segments_kernel<ElemT, OffT, int32_t><<<static_cast<unsigned>(ctas), kPermThreads, 0, stream>>>(
-        static_cast<const ElemT*>(in), static_cast<ElemT*>(out), in_offsets, out_offsets,
-        static_cast<const int32_t*>(perm), num_segments, total);
-  } else {
-    permute_segments_kernel<ElemT, OffT, int64_t><<<static_cast<unsigned>(ctas), kPermThreads, 0, stream>>>(
-        static_cast<const ElemT*>(in), static_cast<ElemT*>(out), in_offsets, out_offsets,
-        static_cast<const int64_t*>(perm), num_segments, total);
+  permute_segments_kernel<ElemT, Elem2T, OffT, PermT, kStarts><<<static_cast<unsigned>(ctas), kPermThreads, 0, stream>>>(
+      static_cast<const ElemT*>(in), static_cast<ElemT*>(out), static_cast<const Elem2T*>(in2),
+      static_cast<Elem2T*>(out2), in_offsets, out_offsets, static_cast<const PermT*>(perm), num_segments, total);
+  return launch_status();
+}
+
+template <typename ElemT>
+int launch_perm_of(const void* in, void* out, const void* in_offsets, const void* out_offsets, const void* perm,
+                   int offset_bytes, int perm_bytes, int64_t num_segments, int64_t total, cudaStream_t stream) {
+  if (offset_bytes == 8)
+    return perm_bytes == 4 ? launch_perm<ElemT, NoElem, int64_t, int32_t, false>(in, out, nullptr, nullptr, in_offsets, out_offsets, perm, num_segments, total, stream)
+                           : launch_perm<ElemT, NoElem, int64_t, int64_t, false>(in, out, nullptr, nullptr, in_offsets, out_offsets, perm, num_segments, total, stream);
+  return perm_bytes == 4 ? launch_perm<ElemT, NoElem, int32_t, int32_t, false>(in, out, nullptr, nullptr, in_offsets, out_offsets, perm, num_segments, total, stream)
+                         : launch_perm<ElemT, NoElem, int32_t, int64_t, false>(in, out, nullptr, nullptr, in_offsets, out_offsets, perm, num_segments, total, stream);
+}
+
+// ---- rows of a [T, B] matrix of lengths as segments ------------------------------------------------
+// A CTA takes one chunk of one row: of an input row, to sum it; of an output row, to copy its lengths.
+constexpr int kLenThreads = 256;
+constexpr int kLenItems = 16;
+constexpr int kLenChunk = kLenThreads * kLenItems;
+
+template <typename LenT, typename PermT>
+__global__ void __launch_bounds__(kLenThreads)
+    permute_lengths_kernel(const LenT* __restrict__ lengths, const PermT* __restrict__ perm,
+                           LenT* __restrict__ permuted, int64_t* __restrict__ chunk_sums, int64_t rows, int64_t cols,
+                           int64_t chunks) {
+  __shared__ int64_t warp_sums[kLenThreads / 32];
+  const int64_t y = blockIdx.x / chunks, chunk = blockIdx.x - y * chunks;
+  const int64_t c0 = chunk * kLenChunk + threadIdx.x;
+  int64_t from = y;
+  if (y >= rows) {
+    from = static_cast<int64_t>(perm[y - rows]);
+    assert(from >= 0 && from < rows);
   }
+  const LenT* src = lengths + from * cols;
+  LenT v[kLenItems];
+#pragma unroll
+  for (int k = 0; k < kLenItems; ++k) {
+    const int64_t c = c0 + k * kLenThreads;
+    v[k] = c < cols ? src[c] : LenT(0);
+  }
+  if (y >= rows) {
+    LenT* dst = permuted + (y - rows) * cols;
+#pragma unroll
+    for (int k = 0; k < kLenItems; ++k) {
+      const int64_t c = c0 + k * kLenThreads;
+      if (c < cols) dst[c] = v[k];
+    }
+    return;
+  }
+  int64_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < kLenItems; ++k) sum += static_cast<int64_t>(v[k]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
+  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kLenThreads / 32; ++w) sum += warp_sums[w];
+    chunk_sums[y * chunks + chunk] = sum;
+  }
+}
+
+constexpr int kRowThreads = 1024;
+
+// Exclusive sum over the CTA's threads; *total is the CTA's sum.
+__device__ __forceinline__ int64_t exclusive_sum(int64_t v, int64_t* total) {
+  __shared__ int64_t warp_sums[kRowThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t up = __shfl_up_sync(kFullMask, incl, o);
+    if (lane >= o) incl += up;
+  }
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  const int64_t sum = warp_sums[lane];
+  int64_t before = lane < warp ? sum : 0, all = sum;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    before += __shfl_xor_sync(kFullMask, before, o);
+    all += __shfl_xor_sync(kFullMask, all, o);
+  }
+  __syncthreads();   // warp_sums may be written again
+  *total = all;
+  return before + incl - v;
+}
+
+// One CTA: where every input row starts, then where every output row starts and where it comes from.
+template <typename PermT>
+__global__ void __launch_bounds__(kRowThreads)
+    permute_row_starts_kernel(const int64_t* __restrict__ chunk_sums, const PermT* __restrict__ perm,
+                              int64_t* in_offsets, int64_t* __restrict__ in_start, int64_t* __restrict__ out_offsets,
+                              int64_t rows, int64_t chunks, int64_t out_rows) {
+  int64_t carry = 0, total;
+  for (int64_t base = 0; base < rows; base += kRowThreads) {
+    const int64_t r = base + threadIdx.x;
+    int64_t len = 0;
+    if (r < rows)
+      for (int64_t k = 0; k < chunks; ++k) len += chunk_sums[r * chunks + k];
+    const int64_t before = exclusive_sum(len, &total);
+    if (r < rows) in_offsets[r] = carry + before;
+    carry += total;
+  }
+  if (threadIdx.x == 0) in_offsets[rows] = carry;
+  __syncthreads();
+  carry = 0;
+  for (int64_t base = 0; base < out_rows; base += kRowThreads) {
+    const int64_t j = base + threadIdx.x;
+    int64_t len = 0, start = 0;
+    if (j < out_rows) {
+      const int64_t from = static_cast<int64_t>(perm[j]);
+      if (from >= 0 && from < rows) {   // (anything else has ended in the lengths kernel)
+        start = in_offsets[from];
+        len = in_offsets[from + 1] - start;
+      }
+      in_start[j] = start;
+    }
+    const int64_t before = exclusive_sum(len, &total);
+    if (j < out_rows) out_offsets[j] = carry + before;
+    carry += total;
+  }
+  if (threadIdx.x == 0) out_offsets[out_rows] = carry;
+}
+
+int64_t length_chunks(int64_t cols) { return cols > 0 ? (cols + kLenChunk - 1) / kLenChunk : 1; }
+
+template <typename LenT, typename PermT>
+int launch_row_starts(const void* lengths, const void* perm, void* permuted, int64_t* in_start, int64_t* out_offsets,
+                      int64_t rows, int64_t cols, int64_t out_rows, int64_t* scratch, cudaStream_t stream) {
+  const int64_t chunks = length_chunks(cols);
+  const int64_t ctas = (rows + (permuted != nullptr ? out_rows : 0)) * chunks;
+  if (ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
+  int64_t* chunk_sums = scratch + rows + 1;
+  permute_lengths_kernel<LenT, PermT><<<static_cast<unsigned>(ctas), kLenThreads, 0, stream>>>(
+      static_cast<const LenT*>(lengths), static_cast<const PermT*>(perm), static_cast<LenT*>(permuted), chunk_sums, rows,
+      cols, chunks);
+  permute_row_starts_kernel<PermT><<<1, kRowThreads, 0, stream>>>(chunk_sums, static_cast<const PermT*>(perm), scratch,
+                                                                  in_start, out_offsets, rows, chunks, out_rows);
   return launch_status();
 }
 
@@ -213,18 +370,73 @@ extern "C" int b200tbe_permute_segments(const void* in, void* out, const void* i
   if ((offset_bytes != 4 && offset_bytes != 8) || (perm_bytes != 4 && perm_bytes != 8))
     return B200TBE_ERR_BAD_ARG;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const bool o64 = offset_bytes == 8;
   switch (elem_bytes) {
-    case 8:
-      return o64 ? launch_perm<uint64_t, int64_t>(in, out, in_offsets, out_offsets, perm, perm_bytes, num_segments, total_elems, stream)
-                 : launch_perm<uint64_t, int32_t>(in, out, in_offsets, out_offsets, perm, perm_bytes, num_segments, total_elems, stream);
-    case 4:
-      return o64 ? launch_perm<uint32_t, int64_t>(in, out, in_offsets, out_offsets, perm, perm_bytes, num_segments, total_elems, stream)
-                 : launch_perm<uint32_t, int32_t>(in, out, in_offsets, out_offsets, perm, perm_bytes, num_segments, total_elems, stream);
-    case 2:
-      return o64 ? launch_perm<uint16_t, int64_t>(in, out, in_offsets, out_offsets, perm, perm_bytes, num_segments, total_elems, stream)
-                 : launch_perm<uint16_t, int32_t>(in, out, in_offsets, out_offsets, perm, perm_bytes, num_segments, total_elems, stream);
-    default:
-      return B200TBE_ERR_UNSUPPORTED;
+    case 8: return launch_perm_of<uint64_t>(in, out, in_offsets, out_offsets, perm, offset_bytes, perm_bytes, num_segments, total_elems, stream);
+    case 4: return launch_perm_of<uint32_t>(in, out, in_offsets, out_offsets, perm, offset_bytes, perm_bytes, num_segments, total_elems, stream);
+    case 2: return launch_perm_of<uint16_t>(in, out, in_offsets, out_offsets, perm, offset_bytes, perm_bytes, num_segments, total_elems, stream);
+    default: return B200TBE_ERR_UNSUPPORTED;
   }
+}
+
+extern "C" size_t b200tbe_permute_row_starts_scratch_bytes(int64_t rows, int64_t cols) {
+  if (rows < 0 || cols < 0) return 0;
+  return static_cast<size_t>(rows + 1 + rows * length_chunks(cols)) * 8;
+}
+
+extern "C" int b200tbe_permute_row_starts(const void* lengths, const void* perm, void* permuted_lengths,
+                                          int64_t* in_start, int64_t* out_offsets, int64_t rows, int64_t cols,
+                                          int64_t out_rows, int32_t length_bytes, int32_t perm_bytes, void* scratch,
+                                          size_t scratch_bytes, b200tbe_stream_t stream_) {
+  if (rows < 0 || cols < 0 || out_rows < 0 || (rows == 0 && out_rows > 0)) return B200TBE_ERR_BAD_ARG;
+  if ((length_bytes != 4 && length_bytes != 8) || (perm_bytes != 4 && perm_bytes != 8)) return B200TBE_ERR_BAD_ARG;
+  if (out_offsets == nullptr || (out_rows > 0 && (in_start == nullptr || perm == nullptr)) ||
+      (rows > 0 && cols > 0 && lengths == nullptr))
+    return B200TBE_ERR_BAD_ARG;
+  if (scratch == nullptr || scratch_bytes < b200tbe_permute_row_starts_scratch_bytes(rows, cols) ||
+      !aligned_to(scratch, 8))
+    return B200TBE_ERR_SCRATCH;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (rows == 0)
+    return cudaMemsetAsync(out_offsets, 0, 8, stream) == cudaSuccess ? B200TBE_OK : B200TBE_ERR_LAUNCH;
+  int64_t* words = static_cast<int64_t*>(scratch);
+  if (length_bytes == 8)
+    return perm_bytes == 8 ? launch_row_starts<int64_t, int64_t>(lengths, perm, permuted_lengths, in_start, out_offsets, rows, cols, out_rows, words, stream)
+                           : launch_row_starts<int64_t, int32_t>(lengths, perm, permuted_lengths, in_start, out_offsets, rows, cols, out_rows, words, stream);
+  return perm_bytes == 8 ? launch_row_starts<int32_t, int64_t>(lengths, perm, permuted_lengths, in_start, out_offsets, rows, cols, out_rows, words, stream)
+                         : launch_row_starts<int32_t, int32_t>(lengths, perm, permuted_lengths, in_start, out_offsets, rows, cols, out_rows, words, stream);
+}
+
+namespace b200tbe {
+namespace {
+template <typename ElemT, typename Elem2T>
+int move_rows(const void* in, void* out, const void* in2, void* out2, const int64_t* in_start, const int64_t* out_offsets,
+              int64_t rows, int64_t total, cudaStream_t stream) {
+  return launch_perm<ElemT, Elem2T, int64_t, int32_t, true>(in, out, in2, out2, in_start, out_offsets, nullptr, rows, total,
+                                                           stream);
+}
+}  // namespace
+}  // namespace b200tbe
+
+extern "C" int b200tbe_permute_rows(const void* in, void* out, int32_t elem_bytes, const void* in2, void* out2,
+                                    int32_t elem2_bytes, const int64_t* in_start, const int64_t* out_offsets,
+                                    int64_t out_rows, int64_t total_elems, b200tbe_stream_t stream_) {
+  if (out_rows < 0 || total_elems < 0) return B200TBE_ERR_BAD_ARG;
+  if (out_rows == 0 || total_elems == 0) return B200TBE_OK;
+  if (in == nullptr || out == nullptr || in_start == nullptr || out_offsets == nullptr || (in2 == nullptr) != (out2 == nullptr))
+    return B200TBE_ERR_BAD_ARG;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  const int second = in2 != nullptr ? elem2_bytes : 0;
+  switch (elem_bytes * 16 + second) {
+    case 8 * 16: return move_rows<uint64_t, NoElem>(in, out, nullptr, nullptr, in_start, out_offsets, out_rows, total_elems, stream);
+    case 4 * 16: return move_rows<uint32_t, NoElem>(in, out, nullptr, nullptr, in_start, out_offsets, out_rows, total_elems, stream);
+    case 2 * 16: return move_rows<uint16_t, NoElem>(in, out, nullptr, nullptr, in_start, out_offsets, out_rows, total_elems, stream);
+    case 8 * 16 + 4: return move_rows<uint64_t, uint32_t>(in, out, in2, out2, in_start, out_offsets, out_rows, total_elems, stream);
+    case 4 * 16 + 4: return move_rows<uint32_t, uint32_t>(in, out, in2, out2, in_start, out_offsets, out_rows, total_elems, stream);
+    default: break;
+  }
+  if (second == 0) return B200TBE_ERR_UNSUPPORTED;
+  // any other pair of widths: one array after the other
+  const int st = b200tbe_permute_rows(in, out, elem_bytes, nullptr, nullptr, 0, in_start, out_offsets, out_rows, total_elems, stream_);
+  if (st != B200TBE_OK) return st;
+  return b200tbe_permute_rows(in2, out2, second, nullptr, nullptr, 0, in_start, out_offsets, out_rows, total_elems, stream_);
 }
