@@ -416,34 +416,45 @@ int64_t sort_plan_max_tiles(int64_t n, int64_t num_segments) {
   return n / kSortPlanTile + (num_segments > 0 ? num_segments : 0) + 1;
 }
 
+bool sort_plan_fits(int64_t max_tiles) { return max_tiles <= 0x7fffffff / kMaxRadix; }
+
 size_t sort_plan_bytes(int64_t n, int64_t num_segments) {
   const int64_t tiles = sort_plan_max_tiles(n, num_segments);
   return 2 * align256(static_cast<size_t>(num_segments + 1) * 4) + align256(static_cast<size_t>(tiles) * sizeof(uint4)) + 256;
+}
+
+SortPlanMem sort_plan_mem(int64_t n, int64_t num_segments, void* plan_mem) {
+  const int64_t tiles = sort_plan_max_tiles(n, num_segments);
+  char* at = static_cast<char*>(plan_mem);
+  auto take = [&](size_t bytes) {
+    char* here = at;
+    at += align256(bytes);
+    return here;
+  };
+  SortPlanMem m{};
+  m.seg_start = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(num_segments + 1) * 4));
+  m.seg_tile_base = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(num_segments + 1) * 4));
+  m.tile_desc = reinterpret_cast<uint4*>(take(static_cast<size_t>(tiles) * sizeof(uint4)));
+  m.total_tiles = reinterpret_cast<uint32_t*>(at);
+  return m;
 }
 
 int build_sort_plan(const void* offsets, int offset_bytes, int num_segments, int64_t stride, int64_t n,
                     void* plan_mem, int32_t* status, SortPlan* plan, const uint32_t** seg_start_out,
                     cudaStream_t stream) {
   const int64_t tiles = sort_plan_max_tiles(n, num_segments);
-  if (tiles > 0x7fffffff / kMaxRadix || num_segments < 1) return B200TBE_ERR_TOO_LARGE;
-  char* at = static_cast<char*>(plan_mem);
-  uint32_t* seg_start = reinterpret_cast<uint32_t*>(at);
-  at += align256(static_cast<size_t>(num_segments + 1) * 4);
-  uint32_t* seg_tile_base = reinterpret_cast<uint32_t*>(at);
-  at += align256(static_cast<size_t>(num_segments + 1) * 4);
-  uint4* tile_desc = reinterpret_cast<uint4*>(at);
-  at += align256(static_cast<size_t>(tiles) * sizeof(uint4));
-  uint32_t* total_tiles = reinterpret_cast<uint32_t*>(at);
+  if (!sort_plan_fits(tiles) || num_segments < 1) return B200TBE_ERR_TOO_LARGE;
+  const SortPlanMem mem = sort_plan_mem(n, num_segments, plan_mem);
   plan_segments_kernel<<<1, kScanThreads, 0, stream>>>(offsets, offset_bytes, num_segments, stride, n,
-                                                      static_cast<int>(tiles), seg_start, seg_tile_base,
-                                                      total_tiles, status);
+                                                      static_cast<int>(tiles), mem.seg_start, mem.seg_tile_base,
+                                                      mem.total_tiles, status);
   plan_tiles_kernel<<<static_cast<unsigned>((tiles + 255) / 256), 256, 0, stream>>>(
-      seg_start, seg_tile_base, num_segments, total_tiles, tile_desc);
-  plan->tile_desc = tile_desc;
-  plan->seg_tile_base = seg_tile_base;
-  plan->total_tiles = total_tiles;
+      mem.seg_start, mem.seg_tile_base, num_segments, mem.total_tiles, mem.tile_desc);
+  plan->tile_desc = mem.tile_desc;
+  plan->seg_tile_base = mem.seg_tile_base;
+  plan->total_tiles = mem.total_tiles;
   plan->max_tiles = static_cast<int>(tiles);
-  if (seg_start_out != nullptr) *seg_start_out = seg_start;
+  if (seg_start_out != nullptr) *seg_start_out = mem.seg_start;
   return launch_status();
 }
 

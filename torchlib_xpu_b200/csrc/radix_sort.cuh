@@ -36,6 +36,16 @@ size_t radix_sort_planned_scratch_bytes(int64_t max_tiles);
 int64_t sort_plan_max_tiles(int64_t n, int64_t num_segments);
 size_t sort_plan_bytes(int64_t n, int64_t num_segments);
 
+// Where the parts of a plan lie in plan_mem (sort_plan_bytes, 256-byte aligned).
+struct SortPlanMem {
+  uint32_t* seg_start;       // [segments + 1]
+  uint32_t* seg_tile_base;   // [segments + 1]
+  uint4* tile_desc;          // [max_tiles]
+  uint32_t* total_tiles;
+};
+SortPlanMem sort_plan_mem(int64_t n, int64_t num_segments, void* plan_mem);
+bool sort_plan_fits(int64_t max_tiles);   // the sort's counts of so many tiles are numbered in 31 bits
+
 // Builds the plan on the device from segment boundaries offsets[s * stride], s = 0..num_segments
 // (int32 or int64, clamped to [0, n]) into plan_mem (sort_plan_bytes, 256-byte aligned). Two small
 // kernels, no host read. *seg_start_out receives the device array [num_segments + 1] of boundaries.

@@ -20,6 +20,8 @@
 //               a second kernel streams each chunk into a partial row in scratch and a third adds a
 //               run's partials in chunk order and applies the update.
 // Summation order is fixed by the data alone on both paths.
+#include <cooperative_groups.h>
+
 #include "radix_sort.cuh"
 #include "scan.cuh"
 #include "tbe_bags.cuh"
@@ -76,7 +78,6 @@ struct BwdDev {
   int32_t max_D;
   // sweep path: the plan (tables -> tiles -> spans)
   const uint32_t* seg_start;       // [T + 1] first sorted position of each table
-  const uint32_t* seg_tile_base;   // [T + 1] first tile of each table
   const uint32_t* total_tiles;     // tiles in use
   const uint4* tile_desc;          // [max_tiles] {begin, count, table, first tile of the table}
   uint32_t* span_flags;            // [max_tiles * spans per tile]
@@ -760,6 +761,8 @@ __global__ void __launch_bounds__(kBwdThreads) finish_long_runs_kernel(BwdDev p)
   }
 }
 
+#include "tbe_backward_small.cuh"
+
 size_t align256(size_t x) { return (x + 255) & ~size_t{255}; }
 
 // Rows of up to kSweepMaxD elements take the sweep path, wider ones the ring engine.
@@ -965,32 +968,51 @@ int run_backward_sweep(BwdDev d, const b200tbe_backward_params* p, const Scratch
   if (key_bits < 1) key_bits = 1;
 
   // the lookups of table t are positions [offsets[t * B], offsets[(t + 1) * B])
-  SortPlan plan{};
-  const uint32_t* seg_start = nullptr;
-  int st = build_sort_plan(p->offsets, p->index_bytes, p->T, p->B, n, scratch + L.plan, p->status, &plan,
-                           &seg_start, stream);
-  if (st != B200TBE_OK) return st;
-  const int64_t bags = static_cast<int64_t>(p->T) * p->B;
-  const int64_t lin_ctas = (bags + 32 * kBwdWarps - 1) / (32 * kBwdWarps);
-  if (lin_ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
-  if (weighted) {
-    linearize_rows_kernel<IndexT, true>
-        <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a);
+  if (!sort_plan_fits(L.max_tiles)) return B200TBE_ERR_TOO_LARGE;
+  if (n <= kSmallSortMax) {
+    SmallSort s{};
+    s.keys[0] = keys_a;
+    s.keys[1] = keys_b;
+    s.vals[0] = vals_a;
+    s.vals[1] = vals_b;
+    const SortPlanMem mem = sort_plan_mem(n, p->T, scratch + L.plan);
+    s.seg_start = mem.seg_start;
+    s.total_tiles = mem.total_tiles;
+    s.tile_desc = mem.tile_desc;
+    s.max_tiles = max_tiles;
+    s.key_bits = key_bits;
+    int result = 0;
+    const int st = launch_small_sort<IndexT>(d, s, weighted, &result, stream);
+    if (st != B200TBE_OK) return st;
+    d.sorted_keys = s.keys[result];
+    d.sorted_vals = s.vals[result];
+    d.seg_start = mem.seg_start;
+    d.total_tiles = mem.total_tiles;
+    d.tile_desc = mem.tile_desc;
   } else {
-    linearize_rows_kernel<IndexT, false>
-        <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a);
+    SortPlan plan{};
+    int st = build_sort_plan(p->offsets, p->index_bytes, p->T, p->B, n, scratch + L.plan, p->status, &plan,
+                             &d.seg_start, stream);
+    if (st != B200TBE_OK) return st;
+    const int64_t bags = static_cast<int64_t>(p->T) * p->B;
+    const int64_t lin_ctas = (bags + 32 * kBwdWarps - 1) / (32 * kBwdWarps);
+    if (lin_ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
+    if (weighted) {
+      linearize_rows_kernel<IndexT, true>
+          <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a);
+    } else {
+      linearize_rows_kernel<IndexT, false>
+          <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a);
+    }
+    bool in_b = false;
+    st = radix_sort_pairs_planned(keys_a, vals_a, keys_b, vals_b, n, key_bits, kSweepSortDigitBits, plan,
+                                  scratch + L.sort, radix_sort_planned_scratch_bytes(max_tiles), &in_b, stream);
+    if (st != B200TBE_OK) return st;
+    d.sorted_keys = in_b ? keys_b : keys_a;
+    d.sorted_vals = in_b ? vals_b : vals_a;
+    d.total_tiles = plan.total_tiles;
+    d.tile_desc = plan.tile_desc;
   }
-  bool in_b = false;
-  st = radix_sort_pairs_planned(keys_a, vals_a, keys_b, vals_b, n, key_bits, kSweepSortDigitBits,
-                                          plan, scratch + L.sort, radix_sort_planned_scratch_bytes(max_tiles),
-                                          &in_b, stream);
-  if (st != B200TBE_OK) return st;
-  d.sorted_keys = in_b ? keys_b : keys_a;
-  d.sorted_vals = in_b ? vals_b : vals_a;
-  d.seg_start = seg_start;
-  d.seg_tile_base = plan.seg_tile_base;
-  d.total_tiles = plan.total_tiles;
-  d.tile_desc = plan.tile_desc;
   d.span_flags = reinterpret_cast<uint32_t*>(scratch + L.span_flags);
   d.span = L.span;
 
