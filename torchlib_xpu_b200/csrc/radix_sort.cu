@@ -45,13 +45,16 @@ struct TilePlace {
   int64_t col;     // index of digit 0's count
   int64_t stride;  // distance between consecutive digits' counts
   bool live;
+  uint32_t seg_begin;            // first key of the segment
+  int seg_first, seg_tiles;      // its tiles
 };
 
+// (by_tile: counts[tile][digit], for sum_counts).
 template <int kTile>
-__device__ __forceinline__ TilePlace place_tile(int64_t n, int radix, int num_tiles, const uint4* desc,
+__device__ __forceinline__ TilePlace place_tile(bool by_tile, int64_t n, int radix, int num_tiles, const uint4* desc,
                                                 const uint32_t* seg_tile_base,
                                                 const uint32_t* total_tiles) {
-  TilePlace t;
+  TilePlace t{};
   if (desc == nullptr) {
     t.base = static_cast<int64_t>(blockIdx.x) * kTile;
     t.tile_n = n - t.base < kTile ? static_cast<int>(n - t.base) : kTile;
@@ -65,12 +68,15 @@ __device__ __forceinline__ TilePlace place_tile(int64_t n, int radix, int num_ti
   const uint4 d = __ldg(desc + blockIdx.x);  // {begin, count, segment, first tile of the segment}
   t.base = d.x;
   t.tile_n = static_cast<int>(d.y);
-  t.stride = __ldg(seg_tile_base + d.z + 1) - d.w;
-  t.col = static_cast<int64_t>(radix) * d.w + (blockIdx.x - d.w);
+  t.seg_first = static_cast<int>(d.w);
+  t.seg_tiles = static_cast<int>(__ldg(seg_tile_base + d.z + 1) - d.w);
+  t.seg_begin = d.x - (blockIdx.x - d.w) * kTile;
+  t.stride = by_tile ? 1 : t.seg_tiles;
+  t.col = by_tile ? static_cast<int64_t>(radix) * blockIdx.x : static_cast<int64_t>(radix) * d.w + (blockIdx.x - d.w);
   return t;
 }
 
-template <typename KeyT>
+template <typename KeyT, bool kSum>
 __global__ void __launch_bounds__(kSortThreads)
     sort_histogram_kernel(const KeyT* __restrict__ keys, int64_t n, int shift, uint32_t mask,
                           int radix, uint32_t* __restrict__ counts, int num_tiles,
@@ -79,7 +85,7 @@ __global__ void __launch_bounds__(kSortThreads)
   constexpr int kItems = SortTile<KeyT>::kItems;
   constexpr int kTile = SortTile<KeyT>::kTile;
   __shared__ uint32_t hist[kMaxRadix];
-  const TilePlace tp = place_tile<kTile>(n, radix, num_tiles, desc, seg_tile_base, total_tiles);
+  const TilePlace tp = place_tile<kTile>(kSum, n, radix, num_tiles, desc, seg_tile_base, total_tiles);
   if (!tp.live) return;
   // all of the thread's keys are requested before the first is counted
   KeyT k[kItems];
@@ -99,12 +105,39 @@ __global__ void __launch_bounds__(kSortThreads)
   for (int d = threadIdx.x; d < radix; d += kSortThreads) counts[d * tp.stride + tp.col] = hist[d];
 }
 
+// The counts of one digit in the tiles of this tile's segment, summed over the tiles before this one and over
+// all of them. Where segments have few tiles this takes the place of the scan: the counts are stored tile by
+// tile (a tile's digits together), a thread adds up one digit's, and two launches a pass do instead of five:
+// 0.63 M pairs in 14 segments, three passes, 90 us with the gaps between launches before, 50 now.
+struct DigitCounts {
+  uint32_t before, all;
+};
+__device__ __forceinline__ DigitCounts sum_counts(const uint32_t* __restrict__ counts, const TilePlace& tp, int radix) {
+  DigitCounts c{0u, 0u};
+  if (static_cast<int>(threadIdx.x) >= radix) return c;
+  const uint32_t* at = counts + static_cast<int64_t>(tp.seg_first) * radix + threadIdx.x;
+  const int mine = static_cast<int>(blockIdx.x) - tp.seg_first;
+  constexpr int kBatch = 16;
+  for (int q0 = 0; q0 < tp.seg_tiles; q0 += kBatch) {
+    uint32_t v[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) v[u] = q0 + u < tp.seg_tiles ? __ldg(at + (q0 + u) * radix) : 0u;
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      c.all += v[u];
+      if (q0 + u < mine) c.before += v[u];
+    }
+  }
+  return c;
+}
+
 // Shared memory of the scatter kernel: per-warp digit counters (16 bits are enough: a warp holds
 // at most 32 * kItems keys, a tile at most 4096), the tile-level digit offsets, and the staging
 // area in which the tile is reordered. Once the tile is staged the counters are dead and their
 // space holds the per-digit distance from staging position to global position. For 4-byte keys:
-// 38 KB with 256 digits (five CTAs per SM at 48 registers: 0.5 % faster than four at 64), 52 KB
-// with 1024 (four), 72 KB with 2048 (three).
+// 38 KB with 256 digits, 52 KB with 1024, 72 KB with 2048 (four, four and three CTAs per SM; with 256
+// digits five fit at 48 registers a thread, but the keys and ranks then spill: 3 passes over 26.7 M pairs
+// 400 us, 386 with four).
 template <typename KeyT, int kRadix>
 struct ScatterSmem {
   union {
@@ -116,9 +149,11 @@ struct ScatterSmem {
   uint32_t vals[SortTile<KeyT>::kTile];
 };
 
-// kRadix: capacity of the digit tables (>= radix, a multiple of kSortThreads). kFull: the tile holds
-// kTile keys (every tile but a segment's last), so no step tests a position against the tile's end.
-template <typename KeyT, int kRadix, bool kFull>
+// kRadix: capacity of the digit tables (>= radix, a multiple of kSortThreads). kBits: bits ranked (>= those
+// of the pass's digit, the ones above are zero); the votes are a third of the kernel's instructions, so
+// passes of 7 and 6 bits vote 7 and 6 times. kFull: the tile holds kTile keys (every tile but a segment's
+// last), so no step tests a position against the tile's end. kSum: see sum_counts.
+template <typename KeyT, int kRadix, int kBits, bool kFull, bool kSum>
 __device__ __forceinline__ void scatter_tile(ScatterSmem<KeyT, kRadix>& sm, const TilePlace& tp,
                                              const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                                              KeyT* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
@@ -127,7 +162,6 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<KeyT, kRadix>& sm, cons
   constexpr int kItems = SortTile<KeyT>::kItems;
   constexpr int kTile = SortTile<KeyT>::kTile;
   constexpr int kDigitsPerThread = kRadix / kSortThreads;
-  constexpr int kBits = kRadix == 256 ? 8 : (kRadix == 1024 ? 10 : 11);   // bits above the pass's digit are zero
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   {
     uint32_t* z = reinterpret_cast<uint32_t*>(&sm.warp_hist[0][0]);
@@ -146,14 +180,16 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<KeyT, kRadix>& sm, cons
     const int it = warp_base + r * 32 + lane;
     k[r] = (kFull || it < tile_n) ? keys_in[base + it] : KeyT(0);
   }
+  DigitCounts seg{};
+  if (kSum) seg = sum_counts(positions, tp, radix);
   __syncthreads();
 
-  uint32_t rank[kItems];
+  // ranks inside the warp, two to a register: sixteen keys, as many payloads in flight and separate ranks spill
+  uint32_t rank[kItems / 2];
 #pragma unroll
   for (int r = 0; r < kItems; ++r) {
     const int it = warp_base + r * 32 + lane;
     const bool valid = kFull || it < tile_n;
-    rank[r] = 0;
     const uint32_t d = static_cast<uint32_t>(k[r] >> shift) & mask;
     // lanes holding the same digit, found one bit at a time with warp votes
     uint32_t peers = kFull ? kFullMask : __ballot_sync(kFullMask, valid);
@@ -167,7 +203,8 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<KeyT, kRadix>& sm, cons
     // value from that lane to its peers with a shuffle over the peers' mask makes the warp run the
     // shuffle once per distinct digit, twenty-odd times.)
     const uint32_t before = sm.warp_hist[warp][d];
-    rank[r] = before + __popc(peers & lanemask_lt);
+    const uint32_t my_rank = before + __popc(peers & lanemask_lt);   // < 32 * kItems
+    rank[r / 2] = r & 1 ? rank[r / 2] | (my_rank << 16) : my_rank;
     __syncwarp();
     if (valid && (peers & lanemask_lt) == 0) sm.warp_hist[warp][d] = static_cast<uint16_t>(before + __popc(peers));
     __syncwarp();
@@ -193,12 +230,15 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<KeyT, kRadix>& sm, cons
   }
   uint32_t unused_total;
   uint32_t start = block_exclusive_scan(thread_total, &unused_total);
+  uint32_t seg_start = 0;
+  if (kSum) seg_start = tp.seg_begin + block_exclusive_scan(seg.all, &unused_total);
 #pragma unroll
   for (int j = 0; j < kDigitsPerThread; ++j) {
     const int d = threadIdx.x * kDigitsPerThread + j;
     sm.digit_start[d] = start;
     // global position of the tile's first key of digit d, minus its staging position
-    totals[j] = (d < radix ? positions[d * tp.stride + tp.col] : 0u) - start;
+    const uint32_t at = kSum ? seg_start + seg.before : (d < radix ? positions[d * tp.stride + tp.col] : 0u);
+    totals[j] = at - start;
     start += run_total[j];
   }
   __syncthreads();
@@ -208,7 +248,8 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<KeyT, kRadix>& sm, cons
     const int it = warp_base + r * 32 + lane;
     if (kFull || it < tile_n) {
       const uint32_t d = static_cast<uint32_t>(k[r] >> shift) & mask;
-      const uint32_t pos = sm.digit_start[d] + sm.warp_hist[warp][d] + rank[r];
+      const uint32_t my_rank = r & 1 ? rank[r / 2] >> 16 : rank[r / 2] & 0xffffu;
+      const uint32_t pos = sm.digit_start[d] + sm.warp_hist[warp][d] + my_rank;
       sm.keys[pos] = k[r];
       sm.vals[pos] = vals_in[base + it];
     }
@@ -238,8 +279,8 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<KeyT, kRadix>& sm, cons
   }
 }
 
-template <typename KeyT, int kRadix>
-__global__ void __launch_bounds__(kSortThreads, kRadix > 1024 ? 3 : (kRadix > 256 ? 4 : 5))
+template <typename KeyT, int kRadix, int kBits, bool kSum>
+__global__ void __launch_bounds__(kSortThreads, kRadix > 1024 ? 3 : 4)
     sort_scatter_kernel(const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                         KeyT* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n,
                         int shift, uint32_t mask, int radix,
@@ -249,12 +290,12 @@ __global__ void __launch_bounds__(kSortThreads, kRadix > 1024 ? 3 : (kRadix > 25
   constexpr int kTile = SortTile<KeyT>::kTile;
   extern __shared__ __align__(16) unsigned char sort_smem[];
   ScatterSmem<KeyT, kRadix>& sm = *reinterpret_cast<ScatterSmem<KeyT, kRadix>*>(sort_smem);
-  const TilePlace tp = place_tile<kTile>(n, radix, num_tiles, desc, seg_tile_base, total_tiles);
+  const TilePlace tp = place_tile<kTile>(kSum, n, radix, num_tiles, desc, seg_tile_base, total_tiles);
   if (!tp.live) return;
   if (tp.tile_n == kTile) {
-    scatter_tile<KeyT, kRadix, true>(sm, tp, keys_in, vals_in, keys_out, vals_out, shift, mask, radix, positions);
+    scatter_tile<KeyT, kRadix, kBits, true, kSum>(sm, tp, keys_in, vals_in, keys_out, vals_out, shift, mask, radix, positions);
   } else {
-    scatter_tile<KeyT, kRadix, false>(sm, tp, keys_in, vals_in, keys_out, vals_out, shift, mask, radix, positions);
+    scatter_tile<KeyT, kRadix, kBits, false, kSum>(sm, tp, keys_in, vals_in, keys_out, vals_out, shift, mask, radix, positions);
   }
 }
 
@@ -333,10 +374,10 @@ struct PassArgs {
   const SortPlan* plan;
 };
 
-template <typename KeyT, int kRadix>
+template <typename KeyT, int kRadix, int kBits, bool kSum>
 int launch_scatter(const KeyT* kin, const uint32_t* vin, KeyT* kout, uint32_t* vout, const PassArgs& a,
                    cudaStream_t stream) {
-  auto kernel = sort_scatter_kernel<KeyT, kRadix>;
+  auto kernel = sort_scatter_kernel<KeyT, kRadix, kBits, kSum>;
   const size_t smem = sizeof(ScatterSmem<KeyT, kRadix>);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
@@ -348,6 +389,20 @@ int launch_scatter(const KeyT* kin, const uint32_t* vin, KeyT* kout, uint32_t* v
       a.plan ? a.plan->total_tiles : nullptr);
   return B200TBE_OK;
 }
+
+template <typename KeyT, bool kSum>
+int launch_scatter_256(const KeyT* kin, const uint32_t* vin, KeyT* kout, uint32_t* vout, const PassArgs& a,
+                       cudaStream_t stream) {
+  if (a.bits <= 6) return launch_scatter<KeyT, 256, 6, kSum>(kin, vin, kout, vout, a, stream);
+  if (a.bits == 7) return launch_scatter<KeyT, 256, 7, kSum>(kin, vin, kout, vout, a, stream);
+  return launch_scatter<KeyT, 256, 8, kSum>(kin, vin, kout, vout, a, stream);
+}
+
+// Segments whose tiles' counts are summed in the scatter kernel rather than scanned: up to this many tiles in
+// all, so a segment with every key in it has no more either. There the two are even: one segment of 1 M keys
+// takes three passes of 18 us scatter and nothing else, or of 12 us and three launches of 7 us; eight segments
+// of 0.67 M keys took 184 us a training step scanned, 149 summed.
+constexpr int64_t kSumTiles = 256;
 
 // plan == nullptr: one flat array of n keys. Otherwise the tiles of the plan (tiles = its bound).
 template <typename KeyT>
@@ -369,20 +424,32 @@ int sort_impl(KeyT* keys_a, uint32_t* vals_a, KeyT* keys_b, uint32_t* vals_b, in
     const uint32_t* vin = in_b ? vals_b : vals_a;
     KeyT* kout = in_b ? keys_a : keys_b;
     uint32_t* vout = in_b ? vals_a : vals_b;
-    sort_histogram_kernel<KeyT><<<tiles, kSortThreads, 0, stream>>>(
+    const PassArgs a{n, shift, bits, tiles, counts, plan};
+    const bool sum = plan != nullptr && bits <= 8 && n / kSortPlanTile <= kSumTiles;
+    if constexpr (sizeof(KeyT) == 4) {   // segments have 4-byte keys
+      if (sum) {
+        sort_histogram_kernel<KeyT, true><<<tiles, kSortThreads, 0, stream>>>(
+            kin, n, shift, mask, radix, counts, tiles, plan->tile_desc, plan->seg_tile_base, plan->total_tiles);
+        const int st = launch_scatter_256<KeyT, true>(kin, vin, kout, vout, a, stream);
+        if (st != B200TBE_OK) return st;
+        in_b = !in_b;
+        shift += bits;
+        continue;
+      }
+    }
+    sort_histogram_kernel<KeyT, false><<<tiles, kSortThreads, 0, stream>>>(
         kin, n, shift, mask, radix, counts, tiles, plan ? plan->tile_desc : nullptr,
         plan ? plan->seg_tile_base : nullptr, plan ? plan->total_tiles : nullptr);
     // with a plan the scan also covers the unused tail of the matrix (tiles is an upper bound);
     // nothing reads it
     int st = exclusive_scan_u32(counts, static_cast<int64_t>(radix) * tiles, tile_sums, nullptr, stream);
     if (st != B200TBE_OK) return st;
-    const PassArgs a{n, shift, bits, tiles, counts, plan};
     if (bits <= 8) {
-      st = launch_scatter<KeyT, 256>(kin, vin, kout, vout, a, stream);
+      st = launch_scatter_256<KeyT, false>(kin, vin, kout, vout, a, stream);
     } else if (bits <= 10) {
-      st = launch_scatter<KeyT, 1024>(kin, vin, kout, vout, a, stream);
+      st = launch_scatter<KeyT, 1024, 10, false>(kin, vin, kout, vout, a, stream);
     } else {
-      st = launch_scatter<KeyT, 2048>(kin, vin, kout, vout, a, stream);
+      st = launch_scatter<KeyT, 2048, 11, false>(kin, vin, kout, vout, a, stream);
     }
     if (st != B200TBE_OK) return st;
     in_b = !in_b;
