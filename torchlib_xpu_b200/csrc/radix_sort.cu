@@ -18,8 +18,7 @@
 // the whole matrix still yields global positions, while keys never leave their segment. Only the
 // bits that differ inside a segment are sorted: 22 bits for tables of 4 M rows however many tables
 // there are.
-#include "radix_sort.cuh"
-#include "scan.cuh"
+#include "sort_plan.cuh"
 
 namespace b200tbe {
 namespace {
@@ -299,67 +298,10 @@ __global__ void __launch_bounds__(kSortThreads, kRadix > 1024 ? 3 : 4)
   }
 }
 
-// ---- plan of a segmented sort -------------------------------------------------------------------
-// seg_start[s] = offsets[s * stride] (clamped to n), seg_tile_base = exclusive prefix of the tiles
-// per segment. One CTA.
 __global__ void __launch_bounds__(kScanThreads)
-    plan_segments_kernel(const void* __restrict__ offsets, int offset_bytes, int num_segments, int64_t stride,
-                         int64_t n, int max_tiles, uint32_t* __restrict__ seg_start,
-                         uint32_t* __restrict__ seg_tile_base, uint32_t* __restrict__ total_tiles,
-                         int32_t* status) {
-  uint32_t carry = 0;
-  auto start_of = [&](int s) -> int64_t {
-    const int64_t i = static_cast<int64_t>(s) * stride;
-    int64_t v = offset_bytes == 8 ? load_index<int64_t>(offsets, i) : load_index<int32_t>(offsets, i);
-    if (v < 0) v = 0;
-    return v > n ? n : v;
-  };
-  for (int base = 0; base <= num_segments; base += kScanThreads) {
-    const int s = base + threadIdx.x;
-    uint32_t tiles = 0;
-    if (s <= num_segments) {
-      const int64_t first = start_of(s);
-      seg_start[s] = static_cast<uint32_t>(first);
-      if (s < num_segments) {
-        const int64_t len = start_of(s + 1) - first;
-        tiles = len > 0 ? static_cast<uint32_t>((len + kSortPlanTile - 1) / kSortPlanTile) : 0u;
-      }
-    }
-    uint32_t total;
-    const uint32_t prefix = block_exclusive_scan(tiles, &total);
-    if (s <= num_segments) seg_tile_base[s] = carry + prefix;
-    carry += total;
-  }
-  if (threadIdx.x == 0) {
-    if (carry > static_cast<uint32_t>(max_tiles)) {   // offsets that do not describe n keys
-      if (status != nullptr) atomicOr(status, B200TBE_DEV_OFFSETS_NOT_MONOTONE);
-      carry = static_cast<uint32_t>(max_tiles);
-    }
-    *total_tiles = carry;
-  }
-}
-
-__global__ void __launch_bounds__(256)
-    plan_tiles_kernel(const uint32_t* __restrict__ seg_start, const uint32_t* __restrict__ seg_tile_base,
-                      int num_segments, const uint32_t* __restrict__ total_tiles,
-                      uint4* __restrict__ tile_desc) {
-  const uint32_t tile = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tile >= *total_tiles) return;
-  // the last segment whose first tile is <= tile (empty segments share their successor's value)
-  int lo = 0, hi = num_segments - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(seg_tile_base + mid) <= tile) {
-      lo = mid;
-    } else {
-      hi = mid - 1;
-    }
-  }
-  const uint32_t first = __ldg(seg_tile_base + lo);
-  const uint32_t begin = __ldg(seg_start + lo) + (tile - first) * kSortPlanTile;
-  const uint32_t end = __ldg(seg_start + lo + 1);
-  const uint32_t count = end - begin < static_cast<uint32_t>(kSortPlanTile) ? end - begin : kSortPlanTile;
-  tile_desc[tile] = make_uint4(begin, count, static_cast<uint32_t>(lo), first);
+    plan_sort_kernel(const void* __restrict__ offsets, int offset_bytes, int num_segments, int64_t stride, int64_t n,
+                     int max_tiles, const SortPlanMem mem, int32_t* status) {
+  plan_sort(offsets, offset_bytes, num_segments, stride, n, max_tiles, mem, status);
 }
 
 template <typename KeyT>
@@ -507,21 +449,13 @@ SortPlanMem sort_plan_mem(int64_t n, int64_t num_segments, void* plan_mem) {
 }
 
 int build_sort_plan(const void* offsets, int offset_bytes, int num_segments, int64_t stride, int64_t n,
-                    void* plan_mem, int32_t* status, SortPlan* plan, const uint32_t** seg_start_out,
-                    cudaStream_t stream) {
+                    void* plan_mem, int32_t* status, SortPlan* plan, cudaStream_t stream) {
   const int64_t tiles = sort_plan_max_tiles(n, num_segments);
   if (!sort_plan_fits(tiles) || num_segments < 1) return B200TBE_ERR_TOO_LARGE;
   const SortPlanMem mem = sort_plan_mem(n, num_segments, plan_mem);
-  plan_segments_kernel<<<1, kScanThreads, 0, stream>>>(offsets, offset_bytes, num_segments, stride, n,
-                                                      static_cast<int>(tiles), mem.seg_start, mem.seg_tile_base,
-                                                      mem.total_tiles, status);
-  plan_tiles_kernel<<<static_cast<unsigned>((tiles + 255) / 256), 256, 0, stream>>>(
-      mem.seg_start, mem.seg_tile_base, num_segments, mem.total_tiles, mem.tile_desc);
-  plan->tile_desc = mem.tile_desc;
-  plan->seg_tile_base = mem.seg_tile_base;
-  plan->total_tiles = mem.total_tiles;
-  plan->max_tiles = static_cast<int>(tiles);
-  if (seg_start_out != nullptr) *seg_start_out = mem.seg_start;
+  plan_sort_kernel<<<1, kScanThreads, 0, stream>>>(offsets, offset_bytes, num_segments, stride, n,
+                                                  static_cast<int>(tiles), mem, status);
+  *plan = sort_plan_of(mem, static_cast<int>(tiles));
   return launch_status();
 }
 
@@ -618,8 +552,7 @@ extern "C" int b200tbe_radix_sort_segments(uint32_t* keys_in, uint32_t* vals_in,
     return B200TBE_ERR_SCRATCH;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   SortPlan plan{};
-  int st = build_sort_plan(seg_offsets, offset_bytes, num_segments, 1, n, scratch, nullptr, &plan, nullptr,
-                           stream);
+  int st = build_sort_plan(seg_offsets, offset_bytes, num_segments, 1, n, scratch, nullptr, &plan, stream);
   if (st != B200TBE_OK) return st;
   char* sort_scratch = static_cast<char*>(scratch) + sort_plan_bytes(n, num_segments);
   bool in_b = false;

@@ -44,15 +44,16 @@ struct SortPlanMem {
   uint32_t* total_tiles;
 };
 SortPlanMem sort_plan_mem(int64_t n, int64_t num_segments, void* plan_mem);
+inline SortPlan sort_plan_of(const SortPlanMem& m, int max_tiles) {
+  return SortPlan{m.tile_desc, m.seg_tile_base, m.total_tiles, max_tiles};
+}
 bool sort_plan_fits(int64_t max_tiles);   // the sort's counts of so many tiles are numbered in 31 bits
 
 // Builds the plan on the device from segment boundaries offsets[s * stride], s = 0..num_segments
-// (int32 or int64, clamped to [0, n]) into plan_mem (sort_plan_bytes, 256-byte aligned). Two small
-// kernels, no host read. *seg_start_out receives the device array [num_segments + 1] of boundaries.
-// Boundaries that describe more than n keys raise B200TBE_DEV_OFFSETS_NOT_MONOTONE in *status.
+// (int32 or int64, clamped to [0, n]) into plan_mem. One small kernel, no host read. Boundaries that
+// describe more than n keys raise B200TBE_DEV_OFFSETS_NOT_MONOTONE in *status.
 int build_sort_plan(const void* offsets, int offset_bytes, int num_segments, int64_t stride, int64_t n,
-                    void* plan_mem, int32_t* status, SortPlan* plan, const uint32_t** seg_start_out,
-                    cudaStream_t stream);
+                    void* plan_mem, int32_t* status, SortPlan* plan, cudaStream_t stream);
 
 // Sorts every segment of the plan by the low key_bits bits of its 4-byte keys, stable, keys never
 // leaving their segment; passes of at most max_digit_bits (<= 11) bits. Buffers ping-pong as above.

@@ -24,6 +24,7 @@
 
 #include "radix_sort.cuh"
 #include "scan.cuh"
+#include "sort_plan.cuh"
 #include "tbe_bags.cuh"
 
 namespace b200tbe {
@@ -969,13 +970,16 @@ int run_backward_sweep(BwdDev d, const b200tbe_backward_params* p, const Scratch
 
   // the lookups of table t are positions [offsets[t * B], offsets[(t + 1) * B])
   if (!sort_plan_fits(L.max_tiles)) return B200TBE_ERR_TOO_LARGE;
+  const SortPlanMem mem = sort_plan_mem(n, p->T, scratch + L.plan);
+  d.seg_start = mem.seg_start;
+  d.total_tiles = mem.total_tiles;
+  d.tile_desc = mem.tile_desc;
   if (n <= kSmallSortMax) {
     SmallSort s{};
     s.keys[0] = keys_a;
     s.keys[1] = keys_b;
     s.vals[0] = vals_a;
     s.vals[1] = vals_b;
-    const SortPlanMem mem = sort_plan_mem(n, p->T, scratch + L.plan);
     s.seg_start = mem.seg_start;
     s.total_tiles = mem.total_tiles;
     s.tile_desc = mem.tile_desc;
@@ -986,32 +990,24 @@ int run_backward_sweep(BwdDev d, const b200tbe_backward_params* p, const Scratch
     if (st != B200TBE_OK) return st;
     d.sorted_keys = s.keys[result];
     d.sorted_vals = s.vals[result];
-    d.seg_start = mem.seg_start;
-    d.total_tiles = mem.total_tiles;
-    d.tile_desc = mem.tile_desc;
   } else {
-    SortPlan plan{};
-    int st = build_sort_plan(p->offsets, p->index_bytes, p->T, p->B, n, scratch + L.plan, p->status, &plan,
-                             &d.seg_start, stream);
-    if (st != B200TBE_OK) return st;
+    const SortPlan plan = sort_plan_of(mem, max_tiles);
     const int64_t bags = static_cast<int64_t>(p->T) * p->B;
-    const int64_t lin_ctas = (bags + 32 * kBwdWarps - 1) / (32 * kBwdWarps);
+    const int64_t lin_ctas = 1 + (bags + 32 * kBwdWarps - 1) / (32 * kBwdWarps);
     if (lin_ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
     if (weighted) {
       linearize_rows_kernel<IndexT, true>
-          <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a);
+          <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a, mem, max_tiles);
     } else {
       linearize_rows_kernel<IndexT, false>
-          <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a);
+          <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a, mem, max_tiles);
     }
     bool in_b = false;
-    st = radix_sort_pairs_planned(keys_a, vals_a, keys_b, vals_b, n, key_bits, kSweepSortDigitBits, plan,
+    const int st = radix_sort_pairs_planned(keys_a, vals_a, keys_b, vals_b, n, key_bits, kSweepSortDigitBits, plan,
                                   scratch + L.sort, radix_sort_planned_scratch_bytes(max_tiles), &in_b, stream);
     if (st != B200TBE_OK) return st;
     d.sorted_keys = in_b ? keys_b : keys_a;
     d.sorted_vals = in_b ? vals_b : vals_a;
-    d.total_tiles = plan.total_tiles;
-    d.tile_desc = plan.tile_desc;
   }
   d.span_flags = reinterpret_cast<uint32_t*>(scratch + L.span_flags);
   d.span = L.span;

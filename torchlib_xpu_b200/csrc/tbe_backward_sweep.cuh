@@ -114,13 +114,19 @@ __device__ __forceinline__ float sqrt_fast(float x) {
 }
 
 // ---- linearize with per-table keys -------------------------------------------------------------
-// As linearize_kernel, but the key is the row id alone: the table is implied by the position.
+// As linearize_kernel, but the key is the row id alone: the table is implied by the position. The first CTA
+// builds the sort's plan meanwhile, which needs two launches (9 us) less than a launch before this one.
 template <typename IndexT, bool kWeighted>
 __global__ void __launch_bounds__(kBwdThreads)
-    linearize_rows_kernel(BwdDev p, int key_bits, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+    linearize_rows_kernel(BwdDev p, int key_bits, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                          const SortPlanMem plan, int max_tiles) {
+  if (blockIdx.x == 0) {
+    plan_sort(p.offsets, static_cast<int>(sizeof(IndexT)), p.T, p.B, p.num_indices, max_tiles, plan, p.status);
+    return;
+  }
   const int lane = threadIdx.x & 31;
   const int64_t total_bags = static_cast<int64_t>(p.T) * p.B;
-  const int64_t bag0 = (static_cast<int64_t>(blockIdx.x) * kBwdWarps + (threadIdx.x >> 5)) * 32;
+  const int64_t bag0 = (static_cast<int64_t>(blockIdx.x - 1) * kBwdWarps + (threadIdx.x >> 5)) * 32;
   if (bag0 >= total_bags) return;
   const int nb = total_bags - bag0 < 32 ? static_cast<int>(total_bags - bag0) : 32;
   const int64_t begin = load_index<IndexT>(p.offsets, bag0);
