@@ -66,3 +66,27 @@ def test_fused_nbit_ops_use_the_fbgemm_op_layout():
         assert np.all(np.abs(back - src) <= scale * 0.51 + 2e-3)
         half = torch.ops.fbgemm.FusedNBitRowwiseQuantizedSBHalfToFloatOrHalf(q, bit_rate, 1)
         assert half.dtype == torch.float16
+
+
+@pytest.mark.parametrize("ty", [oracle.INT8, oracle.INT4, oracle.INT2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("D", [4, 64, 128, 132, 256, 260, 512])
+@pytest.mark.parametrize("header_first", [True, False])
+def test_quantise_vectors_match_the_scalar_kernel(ty, dtype, D, header_first):
+    """The same rows from an address that is not a whole vector take the scalar kernel. Values that round half to
+    even, codes at both ends, rows of one value, infinities and NaN: the same bytes."""
+    rng = workloads.rng_for(610 + D)
+    levels = {oracle.INT8: 255, oracle.INT4: 15, oracle.INT2: 3}[ty]
+    src = rng.uniform(-1, 1, size=(131, D)).astype(np.float32)
+    src[0] = rng.integers(0, 2 * levels + 1, size=D) / 2      # halves between codes: scale 1, bias 0
+    src[0, :2] = 0, levels
+    src[1] = 3.0
+    src[2, 1], src[3, 2], src[4, 3] = np.inf, -np.inf, np.nan
+    src[5] = np.nan
+    src[6] *= 1e-7
+    x = torch.from_numpy(src).to(dtype).cuda()
+    off = torch.empty(x.numel() + 1, dtype=dtype, device="cuda")[1:].view_as(x).copy_(x)
+    assert off.data_ptr() % (4 * x.element_size()) != 0
+    want = cabi.quantize_rows(off, ty, 4, header_first=header_first)
+    got = cabi.quantize_rows(x, ty, 4, header_first=header_first)
+    assert torch.equal(got, want)
