@@ -158,3 +158,43 @@ def test_nbit_groups_of_bags(weighted, pooling, idx_dtype, B):
     want = oracle.nbit_forward(W, wo, tys_a, Do, 16, B, np.where(keep > 0, indices, 0), offsets,
                                keep if psw is None else psw * keep, pooling)
     np.testing.assert_allclose(got.cpu().numpy(), want, rtol=RTOL, atol=ATOL)
+
+
+@pytest.mark.parametrize("D", [16, 32, 48, 64, 96, 112, 128, 144, 256, 272, 512])
+@pytest.mark.parametrize("weighted,pooling,out_dtype,align,B", [
+    (False, oracle.SUM, torch.float32, 16, 29),      # vectors, one bag per warp
+    (True, oracle.MEAN, torch.float16, 16, 12011),   # vectors, groups of two bags, the last group short
+    (False, oracle.MEAN, torch.float32, 8, 29),      # INT4 by vectors, INT8 by words (or the ring engine)
+    (True, oracle.SUM, torch.float32, 4, 29),        # words (or the ring engine)
+])
+def test_nbit_rows_in_vectors_of_sixteen_codes(D, weighted, pooling, out_dtype, align, B):
+    """Rows of 1 to 32 vectors (groups of 2 to 32 lanes, full and with idle lanes), next to rows that are not
+    whole vectors; empty bags (the last ones too), ids out of range, one with an infinite weight."""
+    rng = workloads.rng_for(330 + D)
+    tys, Ds, rows = [oracle.INT8, oracle.INT4, oracle.INT8, oracle.INT4], [D, D, 20, 24], [90, 210, 30, 40]
+    T = len(tys)
+    W, wo, Do, tys_a = helpers.quantised_tables(rng, rows, Ds, tys, align)
+    lengths, _, _ = helpers.ragged_bags(rng, T, B, rows, 0, 9 if B > 100 else 80, empty_fraction=0.2)
+    lengths[B - 3:B] = 0
+    lengths[-2:] = 0
+    offsets = np.zeros(T * B + 1, dtype=np.int64)
+    np.cumsum(lengths, out=offsets[1:])
+    indices = np.concatenate([rng.integers(0, rows[t], size=int(offsets[(t + 1) * B] - offsets[t * B]))
+                              for t in range(T)]).astype(np.int64)
+    bad_at = rng.choice(int(offsets[2 * B]), size=20, replace=False)
+    bad, keep = indices.copy(), np.ones(indices.size, dtype=np.float32)
+    bad[bad_at[:10]], bad[bad_at[10:]], keep[bad_at] = 210, -1, 0.0
+    psw = rng.random(indices.size).astype(np.float32) if weighted else None
+    given = None if psw is None else psw.copy()
+    if weighted and align == 16:
+        given[bad_at[0]] = np.inf
+    got, status = _run(W, wo, tys_a, Do, rows, B, bad, offsets, given, pooling, out_dtype, align, tell_types=B > 100)
+    assert status & cabi.DEV_INDEX_OUT_OF_RANGE
+    want = oracle.nbit_forward(W, wo, tys_a, Do, align, B, np.where(keep > 0, indices, 0), offsets,
+                               keep if psw is None else psw * keep, pooling)
+    got = got.float().cpu().numpy()
+    assert np.isfinite(got).all()
+    if out_dtype == torch.float16:
+        np.testing.assert_allclose(got, want, rtol=RTOL, atol=ATOL)
+    else:   # sums of at most 80 dequantised terms of magnitude about 1, in another order
+        np.testing.assert_allclose(got, want, rtol=1e-5, atol=2e-5)

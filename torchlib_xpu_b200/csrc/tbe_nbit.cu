@@ -1,8 +1,8 @@
 // Quantised-inference TBE forward: INT8 / INT4 / INT2 row-wise quantised tables with an fp16
 // {scale, bias} header per row, plus FP16 / FP32 tables, mixed per table.
 //
-// Two kernels share a call. INT8 and INT4 tables of at most 128 elements per row -- what inference
-// tables are -- go through the register gather of tbe_nbit_bags.cuh (one warp per group of bags, code words
+// Two kernels share a call. INT8 and INT4 tables of at most 128 elements per row (512 where the rows are
+// whole aligned vectors) -- what inference tables are -- go through the register gather of tbe_nbit_bags.cuh (one warp per group of bags, codes
 // fetched straight into registers). Everything else (INT2, float rows, wider rows, rows that are
 // not 4-byte aligned) goes through the streaming gather engine of tbe_stream.cuh, described next;
 // each kernel skips the other's tables.
@@ -43,6 +43,7 @@ struct NbitParams {
   int32_t only_bag_tables;   // the caller vouches that every table is INT8 / INT4: no ring kernel
   int32_t bag_group;         // bags per warp of the register-gather kernel
   int32_t groups_per_table;
+  int32_t by_type;           // tables of one type after those of the other (table_by_type)
 };
 
 __device__ __forceinline__ int64_t round_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
@@ -216,6 +217,9 @@ extern "C" int b200tbe_nbit_forward(const b200tbe_nbit_forward_params* p,
   // types present, when the caller says (bit i: some table has type code i): with INT8 and INT4
   // alone and narrow rows the ring kernel would find nothing to do and is not launched
   const uint32_t fast_types = (1u << B200TBE_INT8) | (1u << B200TBE_INT4);
+  // INT8 beside INT4 or types unknown (one type alone needs no order)
+  d.by_type = p->T > 1 && p->T <= kNbitOrderedTables &&
+              (p->table_type_mask == 0 || (p->table_type_mask & fast_types) == fast_types);
   d.only_bag_tables = p->table_type_mask != 0 && (p->table_type_mask & ~fast_types) == 0 &&
                       p->max_D <= kNbitBagMaxD && p->row_alignment % 4 == 0;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
