@@ -146,8 +146,9 @@ __device__ __forceinline__ void convert_row16(const LumaScale& ls, const LumaSca
   out[2] = make_uint4(w[8], w[9], w[10], w[11]);
 }
 
-// A plain grid, one block of 16 pixels x 2 rows per thread, no shared memory.
-__global__ void __launch_bounds__(kNv12Threads)
+// A plain grid, one block of 16 pixels x 2 rows per thread, no shared memory. Eight CTAs per SM (32
+// registers): a 4K frame is 1013 CTAs, one wave instead of one and a bit (12.31 -> 12.29 us a call).
+__global__ void __launch_bounds__(kNv12Threads, 8)
     nv12_to_rgb_blocks_kernel(const uint8_t* __restrict__ y_plane, const uint8_t* __restrict__ uv_plane,
                               uint8_t* __restrict__ rgb, int width, int height, int stride,
                               bool fullrange, bool tiled) {
@@ -224,3 +225,4 @@ extern "C" int b200tbe_nv12_to_rgb(const uint8_t* y_plane, const uint8_t* uv_pla
   }
   return launch_status();
 }
+
