@@ -400,3 +400,12 @@ def test_backward_small_batch_of_wide_keys():
     hs = np.array([0, rows], dtype=np.int64)
     _check(1, W, wo, Do, offsets, indices, None, grad, hs, np.zeros(rows, dtype=np.float32), B, np.float16, np.float32,
            oracle.SUM, oracle.SGD)
+
+
+@pytest.mark.parametrize("T", [128, 129])
+def test_backward_small_batch_over_many_tables(T):
+    """Up to 128 tables the one-launch sort takes a cluster per table, beyond them the general path sorts."""
+    rng = workloads.rng_for(485)
+    rows, Ds, B = [60] * T, [8] * T, 9
+    case = _backward_case(rng, rows, Ds, B, 0, 6, np.float32, np.float32, oracle.SUM, oracle.ROWWISE_ADAGRAD, True)
+    _check(*case, B, np.float32, np.float32, oracle.SUM, oracle.ROWWISE_ADAGRAD)

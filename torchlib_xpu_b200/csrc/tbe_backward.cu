@@ -974,7 +974,7 @@ int run_backward_sweep(BwdDev d, const b200tbe_backward_params* p, const Scratch
   d.seg_start = mem.seg_start;
   d.total_tiles = mem.total_tiles;
   d.tile_desc = mem.tile_desc;
-  if (n <= kSmallSortMax) {
+  if (n <= kSmallSortMax && p->T <= kSmallSortTables) {
     SmallSort s{};
     s.keys[0] = keys_a;
     s.keys[1] = keys_b;

@@ -215,7 +215,8 @@ int launch_forward(const FwdParams& d, int max_D, cudaStream_t stream) {
   const int64_t max_row = static_cast<int64_t>(max_D) * sizeof(WT);
   if (max_row <= 512) return launch_bags<WT, OT, IndexT>(d, false, stream);
   if (max_row <= kWideRowBytes) return launch_bags<WT, OT, IndexT>(d, true, stream);
-  if (max_D <= 1024) return launch_one<WT, OT, IndexT, 8>(d, stream);
+  if constexpr (sizeof(WT) == 4)   // fp16 rows of up to 1024 elements have at most 2048 bytes
+    if (max_D <= 1024) return launch_one<WT, OT, IndexT, 8>(d, stream);
   return B200TBE_ERR_UNSUPPORTED;
 }
 

@@ -1,14 +1,13 @@
-// Quantised-inference lookup for the common tables: INT8 and INT4 rows of at most 128 elements.
+// Quantised-inference lookup for the common tables: INT8 and INT4 rows of at most 512 elements.
 //
-// One warp per group of consecutive bags in a plain grid, no shared memory. A row is {fp16 scale, fp16 bias} followed by
-// the codes, so the codes start 4 bytes into a 16-byte aligned row: they cannot be fetched with
-// aligned 16-byte vectors without dragging the header and the padding through the arithmetic. They
-// can be fetched as 32-bit words, which is how this kernel reads them: half a warp takes one row,
-// lane w of the half loads code word w (INT8: also word w + 16) and the header word, which all 16
-// lanes read from the same address (one broadcast transaction), so EVERY lane dequantises payload:
-// 8 elements per lane and row for D = 128 in either type. Two rows (one per half-warp) travel
-// through each instruction, several steps' loads are issued before the first is used, and loads
-// allocate in L1, where the head of a skewed id stream stays.
+// One warp per group of consecutive bags in a plain grid, no shared memory. A row is {fp16 scale, fp16 bias}
+// followed by the codes, so the codes start 4 bytes into the row. Rows of whole, aligned vectors of sixteen
+// codes -- nearly all tables -- are fetched in those vectors, which cover the header and all code words but
+// the last; see pool_quantised_vectors. Other rows of at most 128 elements are fetched as 32-bit words
+// (pool_quantised_bags): half a warp takes one row, lane w of the half loads code word w (INT8: also word
+// w + 16) and the header word, which all 16 lanes read from the same address (one broadcast transaction).
+// Either way EVERY lane dequantises payload, several steps' loads are issued before the first is used, and
+// loads allocate in L1, where the head of a skewed id stream stays.
 //
 // Arithmetic per element: the code becomes an exact fp16 integer (byte or nibble dropped into the
 // mantissa of 1024.0, then minus 1024 -- for the nibbles that sit 4 bits up, times 1/16 minus 64),
