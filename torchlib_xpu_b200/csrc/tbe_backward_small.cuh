@@ -21,7 +21,7 @@ constexpr int kSmallItems = 16;                                       // keys pe
 constexpr int kSmallCluster = 8;                                      // CTAs per table
 constexpr int kSmallSortMax = kSmallCluster * kSmallThreads * kSmallItems;   // 65536
 // A table takes a cluster however few lookups it has, and some 37 clusters run at a time: 41 000 lookups over
-// 32 / 64 / 128 tables take 13 / 26 / 49 us, the general path's eight launches about 50.
+// 32 / 64 / 128 tables take 13 / 26 / 49 us, the general path's seven launches about 50.
 constexpr int kSmallSortTables = 128;
 constexpr int kSmallRadix = 256;
 constexpr int kSmallBags = 4096;                                      // bag starts kept in shared memory
