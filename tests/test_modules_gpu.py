@@ -63,3 +63,64 @@ def test_inference_module_quantises_and_pools():
             start, stride = int(mod.weights_offsets[t]), mod.row_strides[t]
             got = W[start:start + r * stride].reshape(r, stride)
             assert np.array_equal(got, oracle.quantize_rows(tables[t], int(ty), 16))
+
+
+def _ones_lookup(rows, ids):
+    """One table of ones, D = 16, one id per bag; the module goes away with the call."""
+    mod = SplitTableBatchedEmbeddingBagsCodegen([(rows, 16)], OptimType.EXACT_SGD, 0.5)
+    mod.weights_dev.data.fill_(1.0)
+    ids = torch.tensor(ids, device="cuda")
+    out = mod(ids, torch.arange(ids.numel() + 1, device="cuda"))
+    out.backward(torch.ones_like(out))
+    return mod.hash_size_cumsum.data_ptr(), out.detach()[:, 0].tolist(), mod.weights_dev.detach()[::16].tolist()
+
+
+def test_row_counts_of_one_module_are_never_those_of_an_earlier_one():
+    """Row counts are remembered between calls. A module built after another one is gone finds its index
+    tables where the other's were, with as many entries: its own counts apply, in the range check of the
+    forward and in the key bits of the backward's sort."""
+    torch.ops.fbgemm.b200tbe_pop_device_status(torch.zeros(1, device="cuda"))
+    reused = 0
+    for small, large in ((3, 200), (5, 7000), (9, 70000)):
+        at, out, _ = _ones_lookup(small, [0, small - 1])
+        assert out == [1.0, 1.0]
+        again, out, weights = _ones_lookup(large, [0, large - 1, small, large - 1])
+        reused += at == again
+        assert out == [1.0] * 4
+        want = [1.0] * large
+        want[0], want[small], want[large - 1] = 0.5, 0.5, 0.0
+        assert weights == want
+    assert reused > 0, "the allocator did not reuse an index table's place: nothing was tested"
+    assert torch.ops.fbgemm.b200tbe_pop_device_status(torch.zeros(1, device="cuda")) == 0
+
+
+def test_row_counts_follow_a_write_to_the_index_table():
+    mod = SplitTableBatchedEmbeddingBagsCodegen([(64, 16)], OptimType.EXACT_SGD, 0.5)
+    mod.weights_dev.data.fill_(1.0)
+    ids, offsets = torch.tensor([0, 40], device="cuda"), torch.arange(3, device="cuda")
+    with torch.no_grad():
+        for rows in (64, 40, 41):
+            mod.hash_size_cumsum.copy_(torch.tensor([0, rows], device="cuda"))
+            assert mod(ids, offsets)[:, 0].tolist() == [1.0, 1.0 if rows > 40 else 0.0]
+    torch.ops.fbgemm.b200tbe_pop_device_status(ids)
+
+
+def test_quantised_row_counts_belong_to_all_that_they_depend_on():
+    """Two modules' tables behind one and the same weights_offsets tensor: the row counts come from the buffer's
+    size, the rows' type and width and their alignment too."""
+    rng = workloads.rng_for(702)
+    specs = [(4, 32, SparseType.INT8), (300, 32, SparseType.INT8), (300, 32, SparseType.INT4), (300, 64, SparseType.INT8)]
+    offsets = torch.arange(2, device="cuda")
+    shared = None
+    torch.ops.fbgemm.b200tbe_pop_device_status(offsets)
+    for rows, dim, ty in specs:
+        mod = IntNBitTableBatchedEmbeddingBagsCodegen([(rows, dim, ty)], output_dtype=SparseType.FP32)
+        tab = rng.uniform(-1, 1, size=(rows, dim)).astype(np.float32)
+        mod.assign_table(0, torch.from_numpy(tab))
+        shared = mod.weights_offsets if shared is None else shared
+        mod.weights_offsets = shared
+        out = mod(torch.tensor([rows - 1], device="cuda"), offsets)
+        want = oracle.nbit_forward(mod.weights_dev.cpu().numpy(), np.zeros(1, np.int64), np.array([int(ty)], np.uint8),
+                                   np.array([0, dim], np.int32), 16, 1, np.array([rows - 1]), np.array([0, 1]))
+        np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-6, atol=1e-6)
+    assert torch.ops.fbgemm.b200tbe_pop_device_status(offsets) == 0

@@ -16,12 +16,17 @@
 // value. There is no CPU implementation and no fallback: only the CUDA dispatch key is registered.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 #include <torch/csrc/autograd/custom_function.h>
 
+#include <algorithm>
+#include <array>
+#include <iterator>
 #include <mutex>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "b200tbe.h"
@@ -72,65 +77,130 @@ int index_bytes_of(const Tensor& indices, const Tensor& offsets) {
 bool is_empty_or_undefined(const Tensor& t) { return !t.defined() || t.numel() == 0; }
 
 // ---- facts about long-lived index tables, read from the device once ----------------------------
-// The lookup ops receive hash_size_cumsum, weights_placements and weights_offsets as DEVICE tensors
-// on every call. What the kernels need from them on the host side (row counts for range checks, the
-// largest table for the sort, "all placements are DEVICE") does not change while the tensor is not
-// written, so it is read back once -- one synchronising copy on the first call -- and remembered
-// under the tensor's storage address, size and version counter.
-struct TensorKey {
-  const void* ptr;
-  int64_t numel;
-  uint64_t version;
-  int device;
-  bool operator==(const TensorKey& o) const {
-    return ptr == o.ptr && numel == o.numel && version == o.version && device == o.device;
+// The lookup ops receive hash_size_cumsum, weights_placements, weights_offsets and the like as DEVICE
+// tensors on every call. What the kernels need from them on the host side (row counts for range checks,
+// the largest table for the sort, "all placements are DEVICE") does not change while the tensors are not
+// written, so it is read back once -- one synchronising copy on the first call -- and remembered for these
+// tensors. An entry holds a weak reference to each tensor's storage: the storage's memory is free to go,
+// but no later storage can be found at its place, so the facts never outlive what they were read from. A
+// write to one of the tensors moves its version counter, and the facts are read again; device tensors among
+// them keep their memory then (renew), since a captured graph may hold on to it.
+
+// A remembered device tensor, and the stream its memory belongs to.
+struct RememberedTensor {
+  Tensor tensor;
+  c10::cuda::CUDAStream stream;
+  // The tensor for a kernel on the current stream: its memory is not handed out again before that kernel ends.
+  const Tensor& here() const {
+    const auto current = c10::cuda::getCurrentCUDAStream(tensor.device().index());
+    if (current != stream) c10::cuda::CUDACachingAllocator::recordStream(tensor.storage().data_ptr(), current);
+    return tensor;
   }
 };
-struct TensorKeyHash {
-  size_t operator()(const TensorKey& k) const {
-    return std::hash<const void*>()(k.ptr) ^ (std::hash<int64_t>()(k.numel) * 31) ^
-           (std::hash<uint64_t>()(k.version) * 131) ^ static_cast<size_t>(k.device);
-  }
-};
-TensorKey key_of(const Tensor& t) {
-  return {t.data_ptr(), t.numel(), static_cast<uint64_t>(t._version()), t.get_device()};
+RememberedTensor remember(const Tensor& t) {
+  return {t, c10::cuda::getCurrentCUDAStream(t.device().index())};
 }
 
-template <typename V>
+struct TableRows {
+  RememberedTensor rows_per_table;   // [T] int64 on the device
+  int64_t max_rows;
+};
+
+// The facts that take the place of older ones about the same tensors.
+bool renew(bool, bool now) { return now; }
+RememberedTensor renew(const RememberedTensor& old, const RememberedTensor& now) {
+  old.here().copy_(now.tensor);
+  c10::cuda::getCurrentCUDAStream(now.tensor.device().index()).synchronize();   // calls on any stream may follow
+  return old;
+}
+TableRows renew(const TableRows& old, const TableRows& now) {
+  return {renew(old.rows_per_table, now.rows_per_table), now.max_rows};
+}
+
+template <typename V, size_t kTensors, size_t kNumbers = 0>
 class FactCache {
  public:
+  // make() may depend on these tensors' contents and on these numbers, and on nothing else.
   template <typename Make>
-  V get(const Tensor& t, Make make) {
-    const TensorKey k = key_of(t);
+  V get(const std::array<const Tensor*, kTensors>& tensors, const std::array<int64_t, kNumbers>& numbers, Make make) {
+    Key key{};
+    std::array<uint64_t, kTensors> versions;
+    for (size_t i = 0; i < kTensors; ++i) {
+      const Tensor& t = *tensors[i];
+      if (!t.is_contiguous() && t.dim() != 1) return make();
+      key.views[i] = {t.storage().unsafeGetStorageImpl(), t.data_ptr(), t.numel(), t.is_contiguous() ? 1 : t.stride(0),
+                      t.scalar_type()};
+      versions[i] = static_cast<uint64_t>(t._version());
+    }
+    key.numbers = numbers;
     {
       std::lock_guard<std::mutex> lock(mu_);
-      auto it = map_.find(k);
-      if (it != map_.end()) return it->second;
+      const auto it = map_.find(key);
+      if (it != map_.end() && it->second.versions == versions) return it->second.facts;
     }
     V v = make();
     std::lock_guard<std::mutex> lock(mu_);
-    if (map_.size() >= 256) map_.clear();   // tables come and go; the facts are cheap to rebuild
-    map_.emplace(k, v);
+    if (map_.size() >= sweep_at_) {   // entries of storages that are gone
+      for (auto it = map_.begin(); it != map_.end();) it = it->second.gone() ? map_.erase(it) : std::next(it);
+      sweep_at_ = std::max<size_t>(256, 2 * map_.size());
+    }
+    const auto old = map_.find(key);
+    if (old != map_.end()) {
+      old->second.versions = versions;
+      return old->second.facts = renew(old->second.facts, v);
+    }
+    Entry e{versions, {}, v};
+    for (const Tensor* t : tensors) e.storages.push_back(t->storage().getWeakStorageImpl());
+    map_.emplace(key, std::move(e));
     return v;
   }
 
  private:
+  struct View {
+    const void* storage;
+    const void* data;
+    int64_t numel, stride;
+    at::ScalarType type;
+    bool operator==(const View& o) const {
+      return storage == o.storage && data == o.data && numel == o.numel && stride == o.stride && type == o.type;
+    }
+  };
+  struct Key {
+    std::array<View, kTensors> views;
+    std::array<int64_t, kNumbers> numbers;
+    bool operator==(const Key& o) const { return views == o.views && numbers == o.numbers; }
+  };
+  struct KeyHash {
+    size_t operator()(const Key& k) const {
+      size_t h = 0;
+      for (const View& v : k.views)
+        h = h * 131 + (std::hash<const void*>()(v.storage) ^ (std::hash<const void*>()(v.data) * 31) ^ static_cast<size_t>(v.numel));
+      for (const int64_t n : k.numbers) h = h * 131 + static_cast<size_t>(n);
+      return h;
+    }
+  };
+  struct Entry {
+    std::array<uint64_t, kTensors> versions;
+    std::vector<c10::weak_intrusive_ptr<c10::StorageImpl>> storages;   // as long as they are held, their addresses are theirs
+    V facts;
+    bool gone() const {
+      for (const auto& s : storages)
+        if (s.expired()) return true;
+      return false;
+    }
+  };
   std::mutex mu_;
-  std::unordered_map<TensorKey, V, TensorKeyHash> map_;
-};
-
-struct TableRows {
-  Tensor rows_per_table;   // [T] int64 on the device
-  int64_t max_rows;
+  std::unordered_map<Key, Entry, KeyHash> map_;
+  size_t sweep_at_ = 256;
 };
 
 TableRows table_rows_of(const Tensor& hash_size_cumsum) {
-  static FactCache<TableRows> cache;
-  return cache.get(hash_size_cumsum, [&] {
+  static FactCache<TableRows, 1> cache;
+  return cache.get({&hash_size_cumsum}, {}, [&] {
     const int64_t n = hash_size_cumsum.numel();
     Tensor rows = (hash_size_cumsum.slice(0, 1, n) - hash_size_cumsum.slice(0, 0, n - 1)).contiguous();
     const int64_t max_rows = n > 1 ? rows.max().item<int64_t>() : 0;
-    return TableRows{rows, max_rows};
+    return TableRows{remember(rows), max_rows};
   });
 }
 
@@ -426,9 +496,9 @@ void check_placements(const Tensor& uvm_weights, const Tensor& lxu_cache_weights
               "uvm_weights must be empty: all tables live in dev_weights (HBM)");
   TORCH_CHECK(is_empty_or_undefined(lxu_cache_weights), "lxu_cache_weights must be empty: no cache");
   if (weights_placements.defined() && weights_placements.numel() > 0) {
-    static FactCache<bool> cache;   // read back once per placements tensor, not once per call
+    static FactCache<bool, 1> cache;   // read back once per placements tensor, not once per call
     const bool all_device = cache.get(
-        weights_placements, [&] { return weights_placements.to(at::kCPU).eq(0).all().item<bool>(); });
+        {&weights_placements}, {}, [&] { return weights_placements.to(at::kCPU).eq(0).all().item<bool>(); });
     TORCH_CHECK(all_device, "weights_placements must be all DEVICE (0)");
   }
 }
@@ -467,7 +537,7 @@ Tensor tbe_forward(const TbeCommon& c) {
   if (c.hash_size_cumsum.defined() && c.hash_size_cumsum.numel() == T + 1 && T > 0) {
     check_cuda_contig(c.hash_size_cumsum, "hash_size_cumsum");
     TORCH_CHECK(c.hash_size_cumsum.scalar_type() == at::kLong, "hash_size_cumsum must be int64");
-    rows_keepalive = table_rows_of(c.hash_size_cumsum).rows_per_table;
+    rows_keepalive = table_rows_of(c.hash_size_cumsum).rows_per_table.here();
     status_word = device_status(c.dev_weights.device());
     p.rows_per_table = rows_keepalive.data_ptr<int64_t>();
     p.status = status_word.data_ptr<int32_t>();
@@ -724,10 +794,11 @@ Tensor int_nbit_split_embedding_codegen_lookup_function(
   // rows_t <= bytes_t / stride_t: an id beyond that would read another table's bytes.
   Tensor rows_keepalive, status_word;
   if (T > 0) {
-    static FactCache<Tensor> cache;
+    static FactCache<RememberedTensor, 3, 3> cache;
     const int64_t total_bytes = dev_weights.numel();
     const int32_t align = p.row_alignment;
-    rows_keepalive = cache.get(weights_offsets, [&] {
+    const RememberedTensor rows_per_table = cache.get(
+        {&weights_offsets, &weights_tys, &D_offsets}, {total_bytes, align, dev_weights.get_device()}, [&] {
       const Tensor wo = weights_offsets.to(at::kCPU), ty = weights_tys.to(at::kCPU), Do = D_offsets.to(at::kCPU);
       Tensor rows = at::empty({T}, at::TensorOptions().dtype(at::kLong));
       for (int64_t t = 0; t < T; ++t) {
@@ -746,8 +817,9 @@ Tensor int_nbit_split_embedding_codegen_lookup_function(
         }
         rows.data_ptr<int64_t>()[t] = stride > 0 && end > begin ? (end - begin) / stride : 0;
       }
-      return rows.to(dev_weights.device());
+      return remember(rows.to(dev_weights.device()));
     });
+    rows_keepalive = rows_per_table.here();
     status_word = device_status(dev_weights.device());
     p.rows_per_table = rows_keepalive.data_ptr<int64_t>();
     p.status = status_word.data_ptr<int32_t>();
