@@ -65,33 +65,46 @@ def test_inference_module_quantises_and_pools():
             assert np.array_equal(got, oracle.quantize_rows(tables[t], int(ty), 16))
 
 
-def _ones_lookup(rows, ids):
-    """One table of ones, D = 16, one id per bag; the module goes away with the call."""
-    mod = SplitTableBatchedEmbeddingBagsCodegen([(rows, 16)], OptimType.EXACT_SGD, 0.5)
-    mod.weights_dev.data.fill_(1.0)
-    ids = torch.tensor(ids, device="cuda")
-    out = mod(ids, torch.arange(ids.numel() + 1, device="cuda"))
-    out.backward(torch.ones_like(out))
-    return mod.hash_size_cumsum.data_ptr(), out.detach()[:, 0].tolist(), mod.weights_dev.detach()[::16].tolist()
+def _table_at(place, values):
+    """A new int64 index table in the memory that a freed one had."""
+    others = []
+    while len(others) < 8192:
+        others.append(torch.tensor(values, device="cuda"))
+        if others[-1].data_ptr() == place:
+            return others[-1]
+    raise AssertionError("the allocator did not hand out the freed table's memory")
 
 
-def test_row_counts_of_one_module_are_never_those_of_an_earlier_one():
-    """Row counts are remembered between calls. A module built after another one is gone finds its index
-    tables where the other's were, with as many entries: its own counts apply, in the range check of the
-    forward and in the key bits of the backward's sort."""
-    torch.ops.fbgemm.b200tbe_pop_device_status(torch.zeros(1, device="cuda"))
-    reused = 0
-    for small, large in ((3, 200), (5, 7000), (9, 70000)):
-        at, out, _ = _ones_lookup(small, [0, small - 1])
-        assert out == [1.0, 1.0]
-        again, out, weights = _ones_lookup(large, [0, large - 1, small, large - 1])
-        reused += at == again
-        assert out == [1.0] * 4
-        want = [1.0] * large
-        want[0], want[small], want[large - 1] = 0.5, 0.5, 0.0
-        assert weights == want
-    assert reused > 0, "the allocator did not reuse an index table's place: nothing was tested"
-    assert torch.ops.fbgemm.b200tbe_pop_device_status(torch.zeros(1, device="cuda")) == 0
+def test_row_counts_of_one_table_are_never_those_of_an_earlier_one():
+    """Row counts are remembered between calls. An index table built after another one was freed lies where that
+    one lay, with as many entries: its own counts apply, in the range check of the forward and in the key bits of
+    the backward's sort."""
+    lookup = torch.ops.fbgemm.split_embedding_codegen_lookup_sgd_function
+    large, D = 70000, 16
+    ids = torch.tensor([0, large - 1, 2, large - 1], device="cuda")
+    offsets = torch.arange(ids.numel() + 1, device="cuda")
+    wo, Do = torch.zeros(1, dtype=torch.int64, device="cuda"), torch.tensor([0, D], dtype=torch.int32, device="cuda")
+    e, ei = torch.empty(0, device="cuda"), torch.empty(0, dtype=torch.int32, device="cuda")
+    torch.ops.fbgemm.b200tbe_pop_device_status(e)
+
+    def step(rows, table):
+        w = torch.ones(large * D, device="cuda")
+        placeholder = torch.zeros(1, device="cuda", requires_grad=True)
+        out = lookup(placeholder, w, e, e, ei, wo, Do, D, D, table, 17, ids.clamp(max=rows - 1), offsets, 0, None, None, ei,
+                     False, 0.0, False, 0.5, 0)
+        out.backward(torch.ones_like(out))
+        return out.detach()[:, 0].tolist(), w[::D]
+
+    first = torch.tensor([0, 3], device="cuda")
+    place = first.data_ptr()
+    assert step(3, first)[0] == [1.0] * 4
+    del first
+    out, w = step(large, _table_at(place, [0, large]))
+    assert out == [1.0] * 4
+    want = torch.ones(large)
+    want[0], want[2], want[large - 1] = 0.5, 0.5, 0.0
+    assert torch.equal(w.cpu(), want)
+    assert torch.ops.fbgemm.b200tbe_pop_device_status(e) == 0
 
 
 def test_row_counts_follow_a_write_to_the_index_table():
