@@ -272,3 +272,45 @@ def test_forward_rows_of_513_to_2048_bytes(wdtype, D, weighted, pooling, idx_dty
                               keep if psw is None else psw * keep, pooling)
     # sums of at most 70 terms of magnitude <= 1 in another order: 70 * 2^-24 of slack
     np.testing.assert_allclose(got.cpu().numpy(), want, rtol=RTOL_FP32, atol=ATOL_FP32_UNIT)
+
+
+def non_finite_weights(rng, offsets, indices, rows, T, B):
+    """Per-sample weights and ids with infinite and NaN weights on ids out of range (a few per table) and on good ids;
+    (ids, weights, weights with the bad ids' set to 0, the bags that hold a good id with such a weight)."""
+    bad, psw = indices.copy(), rng.random(indices.size).astype(np.float32) + 0.5
+    owner = np.repeat(np.arange(T * B), np.diff(offsets))
+    touched = np.zeros(T * B, dtype=bool)
+    kept = psw.copy()
+    for t in range(T):
+        at = int(offsets[t * B]) + rng.choice(int(offsets[(t + 1) * B] - offsets[t * B]), size=16, replace=False)
+        bad[at[:4]], bad[at[4:8]] = -1, rows[t]
+        psw[at[:8]] = kept[at[:8]] = 0.0
+        psw[at[[0, 1, 4, 5]]], psw[at[[2, 6]]] = np.inf, np.nan
+        psw[at[8:12]] = kept[at[8:12]] = np.inf
+        psw[at[12:]] = kept[at[12:]] = np.nan
+        touched[owner[at[8:]]] = True
+    return bad, psw, kept, touched
+
+
+@pytest.mark.parametrize("wdtype", [np.float32, np.float16])
+@pytest.mark.parametrize("Ds", [(4, 8, 16), (32, 64, 128), (24, 200, 256), (512, 16, 64)])
+@pytest.mark.parametrize("idx_dtype,B", [(np.int64, 40), (np.int32, 24000)])   # one bag per warp, groups of bags
+def test_forward_weights_that_are_not_finite_stay_in_their_bags(wdtype, Ds, idx_dtype, B):
+    """A lookup that is skipped adds nothing whatever its weight, and the weight of a good lookup reaches its own bag
+    only: narrow rows (several rounds of a group's rows per 32 ids), wide rows, and narrow rows beside wide ones."""
+    rng = workloads.rng_for(240 + sum(Ds))
+    rows, T = [300, 70, 500], len(Ds)
+    W, wo, Do = helpers.float_tables(rng, rows, Ds, wdtype, -1.0, 1.0)
+    _, offsets, indices = helpers.ragged_bags(rng, T, B, rows, 0, 70 if B < 100 else 9, empty_fraction=0.1)
+    bad, psw, kept, touched = non_finite_weights(rng, offsets, indices, rows, T, B)
+    got, status = _run(W, wo, Do, rows, B, bad, offsets, psw, oracle.SUM, torch.float32, idx_dtype=idx_dtype)
+    assert status & cabi.DEV_INDEX_OUT_OF_RANGE
+    ty = oracle.FP32 if wdtype == np.float32 else oracle.FP16
+    want = oracle.tbe_forward(W, ty, wo, Do, B, indices, offsets, np.where(np.isfinite(kept), kept, 0), oracle.SUM)
+    got = got.cpu().numpy()
+    for t in range(T):
+        clean = ~touched[t * B:(t + 1) * B]
+        # sums of at most 70 terms of magnitude <= 1.5 in another order
+        np.testing.assert_allclose(got[clean, Do[t]:Do[t + 1]], want[clean, Do[t]:Do[t + 1]], rtol=RTOL_FP32,
+                                   atol=1.5 * ATOL_FP32_UNIT)
+        assert not np.isfinite(got[~clean, Do[t]:Do[t + 1]]).any()

@@ -5,6 +5,7 @@ import torch
 
 import oracle
 from tests import helpers
+from tests.test_tbe_forward_gpu import non_finite_weights
 from torchlib_xpu_b200 import cabi, workloads
 
 pytestmark = pytest.mark.gpu
@@ -198,3 +199,24 @@ def test_nbit_rows_in_vectors_of_sixteen_codes(D, weighted, pooling, out_dtype, 
         np.testing.assert_allclose(got, want, rtol=RTOL, atol=ATOL)
     else:   # sums of at most 80 dequantised terms of magnitude about 1, in another order
         np.testing.assert_allclose(got, want, rtol=1e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("D,align", [(128, 4), (64, 4), (24, 16), (128, 16), (32, 16), (256, 16)])
+@pytest.mark.parametrize("B", [40, 12000])   # one bag per warp, groups of bags
+def test_nbit_weights_that_are_not_finite_stay_in_their_bags(D, align, B):
+    """A lookup that is skipped adds nothing whatever its weight, and the weight of a good lookup reaches its own bag
+    only: rows fetched as words and as vectors."""
+    rng = workloads.rng_for(360 + D)
+    tys, rows = [oracle.INT8, oracle.INT4, oracle.INT8], [300, 70, 500]
+    T = len(tys)
+    W, wo, Do, tys_a = helpers.quantised_tables(rng, rows, [D] * T, tys, align)
+    _, offsets, indices = helpers.ragged_bags(rng, T, B, rows, 0, 70 if B < 100 else 9, empty_fraction=0.1)
+    bad, psw, kept, touched = non_finite_weights(rng, offsets, indices, rows, T, B)
+    got, status = _run(W, wo, tys_a, Do, rows, B, bad, offsets, psw, oracle.SUM, torch.float32, align)
+    assert status & cabi.DEV_INDEX_OUT_OF_RANGE
+    want = oracle.nbit_forward(W, wo, tys_a, Do, align, B, indices, offsets, np.where(np.isfinite(kept), kept, 0), oracle.SUM)
+    got = got.cpu().numpy()
+    for t in range(T):
+        clean = ~touched[t * B:(t + 1) * B]
+        # sums of at most 70 dequantised terms of magnitude <= 1.5, in another order
+        np.testing.assert_allclose(got[clean, t * D:(t + 1) * D], want[clean, t * D:(t + 1) * D], rtol=1e-5, atol=3e-5)

@@ -189,10 +189,13 @@ __device__ __forceinline__ void pool_float_bag(const BagLaunch<OT>& p, const cha
       for (int u = 0; u < kLoads; ++u) {
         const int rr = j + u * G + h;
         const uint32_t row = __shfl_sync(kFullMask, my_row, rr & 31);
-        if (kWeighted) w[u] = __shfl_sync(kFullMask, my_w, rr & 31);
+        const bool ok = rr < n && row != kNoRow;
+        if (kWeighted) {
+          w[u] = __shfl_sync(kFullMask, my_w, rr & 31);
+          if (!ok) w[u] = 0.f;   // 0 x infinity: a skipped lookup adds nothing whatever its weight
+        }
         x[u] = make_uint4(0u, 0u, 0u, 0u);  // +0.0 in either type: adding it changes nothing
-        if (rr < n && row != kNoRow && active)
-          x[u] = ldg_cached16(row_address(lane_base, row, static_cast<uint32_t>(row_bytes)));
+        if (ok && active) x[u] = ldg_cached16(row_address(lane_base, row, static_cast<uint32_t>(row_bytes)));
       }
 #pragma unroll
       for (int u = 0; u < kLoads; ++u) {
@@ -359,10 +362,13 @@ __device__ __forceinline__ void pool_float_bags_of(const BagLaunch<OT>& p, const
         for (int u = 0; u < kLoads; ++u) {
           const int rr = j + u * G + h;
           const uint32_t row = __shfl_sync(kFullMask, my_row, rr & 31);
-          if (kWeighted) w[u] = __shfl_sync(kFullMask, my_w, rr & 31);
+          const bool ok = rr < n && row != kNoRow;
+          if (kWeighted) {
+            w[u] = __shfl_sync(kFullMask, my_w, rr & 31);
+            if (!ok) w[u] = 0.f;   // 0 x infinity: a skipped lookup adds nothing whatever its weight
+          }
           x[u] = make_uint4(0u, 0u, 0u, 0u);  // +0.0 in either type: adding it changes nothing
-          if (rr < n && row != kNoRow && active)
-            x[u] = ldg_cached16(row_address(lane_base, row, static_cast<uint32_t>(row_bytes)));
+          if (ok && active) x[u] = ldg_cached16(row_address(lane_base, row, static_cast<uint32_t>(row_bytes)));
         }
       }
       if (c + j + round_rows < cur_end) {        // the whole round inside the open bag, which goes on

@@ -266,7 +266,10 @@ __device__ __forceinline__ void pool_quantised_bags(const NbitParams& p, const c
         w1[u] = 0u;
         if (on0) w0[u] = ldg_cached4(src);
         if (on1) w1[u] = ldg_cached4(src + 64);
-        if (((ok_mask >> rr) & 1u) == 0 || j + 2 * u + half >= 32) hdr[u] = 0u;
+        if (((ok_mask >> rr) & 1u) == 0 || j + 2 * u + half >= 32) {
+          hdr[u] = 0u;
+          if (kWeighted) wt[u] = 0.f;   // (0 x infinity)
+        }
       }
       if (c + j + 2 * kSteps < cur_end) {         // the whole round inside the open bag, which goes on
 #pragma unroll
