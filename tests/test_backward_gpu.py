@@ -409,3 +409,29 @@ def test_backward_small_batch_over_many_tables(T):
     rows, Ds, B = [60] * T, [8] * T, 9
     case = _backward_case(rng, rows, Ds, B, 0, 6, np.float32, np.float32, oracle.SUM, oracle.ROWWISE_ADAGRAD, True)
     _check(*case, B, np.float32, np.float32, oracle.SUM, oracle.ROWWISE_ADAGRAD)
+
+
+@pytest.mark.parametrize("D", [8, 32, 64, 128])
+@pytest.mark.parametrize("gdtype", [np.float32, np.float16])
+def test_backward_weights_that_are_not_finite_stay_with_their_rows(D, gdtype):
+    """Rows looked up once with an infinite or NaN weight, between rows looked up many times: the others' updates
+    are what they would be without."""
+    rng = workloads.rng_for(486 + D)
+    T, W, wo, Do, offsets, indices, _, grad, hs, mom, B = _runs_case(rng, [5, 1, 9, 1, 1, 40] * 30, D, np.float32, 50, "mixed")
+    once = np.flatnonzero(np.bincount(indices) == 1)
+    hit = rng.choice(once, size=60, replace=False)
+    psw = rng.integers(1, 4, size=B).astype(np.float32)
+    kept = psw.copy()
+    at = np.isin(indices, hit)
+    psw[at], kept[at] = rng.choice([np.inf, -np.inf, np.nan], size=60).astype(np.float32), 0.0
+    W_ref, m_ref = W.copy(), mom.copy()
+    oracle.tbe_backward(W_ref, oracle.FP32, wo, Do, hs, B, indices, offsets, grad, m_ref, hs[:-1],
+                        oracle.ROWWISE_ADAGRAD, 0.05, 1e-8, kept)
+    dW, dm = _dev(W), _dev(mom)
+    cabi.backward(dW, _dev(wo), _dev(Do), _dev(hs), int(hs[-1] - 1).bit_length(), D, _dev(indices), _dev(offsets), B,
+                  _dev(grad.astype(gdtype)), oracle.ROWWISE_ADAGRAD, 0.05, 1e-8, dm, _dev(hs[:-1].copy()),
+                  per_sample_weights=_dev(psw))
+    torch.cuda.synchronize()
+    others = np.setdiff1d(np.arange(int(hs[-1])), hit)
+    np.testing.assert_allclose(dW.cpu().numpy().reshape(-1, D)[others], W_ref.reshape(-1, D)[others], rtol=1e-5, atol=1e-6)
+    np.testing.assert_allclose(dm.cpu().numpy()[others], m_ref[others], rtol=1e-5)

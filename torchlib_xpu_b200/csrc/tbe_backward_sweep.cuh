@@ -404,7 +404,10 @@ __device__ __forceinline__ void sweep_span(const BwdDev& p, const SpanCtx& sc, c
         for (int u = 0; u < kSweepLoads; ++u) {
           const uint32_t off = __shfl_sync(kFullMask, goff_sweep, j0 + u, GS);
           mu[u] = 1.f;
-          if (kScaled) mu[u] = __shfl_sync(kFullMask, cur.mult, j0 + u, GS);
+          if (kScaled) {
+            mu[u] = __shfl_sync(kFullMask, cur.mult, j0 + u, GS);
+            if (NG > 1 && off == kNoSlice) mu[u] = 0.f;   // a one-lookup run's weight, should it be infinite, stays with it
+          }
           const char* src = tab.g_lane + (static_cast<uint64_t>(off) << 4);
 #pragma unroll
           for (int c = 0; c < kC; ++c) {
