@@ -61,6 +61,9 @@ typedef enum { B200TBE_OPT_SGD = 0, B200TBE_OPT_ROWWISE_ADAGRAD = 1 } b200tbe_op
 
 /* Bits a kernel may OR into the optional device status word (int32). */
 #define B200TBE_DEV_INDEX_OUT_OF_RANGE 1
+/* b200tbe_backward found offsets that decrease; it has changed nothing. Found: any table that ends before it
+ * begins; any bag that does, from 65 537 lookups on, beyond 128 tables and for rows of more than 512 elements
+ * (in smaller batches such a bag only moves lookups of its table to other bags of the table). */
 #define B200TBE_DEV_OFFSETS_NOT_MONOTONE 2
 #define B200TBE_DEV_UNSUPPORTED_SHAPE 4 /* a table's row is not whole 16-byte vectors */
 #define B200TBE_DEV_WAIT_TIMEOUT 8      /* reserved: a bounded wait inside a kernel gave up (no kernel of

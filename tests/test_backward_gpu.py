@@ -435,3 +435,69 @@ def test_backward_weights_that_are_not_finite_stay_with_their_rows(D, gdtype):
     others = np.setdiff1d(np.arange(int(hs[-1])), hit)
     np.testing.assert_allclose(dW.cpu().numpy().reshape(-1, D)[others], W_ref.reshape(-1, D)[others], rtol=1e-5, atol=1e-6)
     np.testing.assert_allclose(dm.cpu().numpy()[others], m_ref[others], rtol=1e-5)
+
+
+def _disordered(where, T, B, lengths):
+    """Offsets of T * B bags whose table 1 ends before it begins, or with one bag inside a table that does."""
+    offsets = np.zeros(T * B + 1, dtype=np.int64)
+    np.cumsum(lengths, out=offsets[1:])
+    n = int(offsets[-1])
+    if where == "table":
+        offsets[B:2 * B + 1] = np.linspace(n, n // 3, B + 1).astype(np.int64)
+    else:
+        b = B + B // 2
+        offsets[b] = offsets[2 * B] + 7   # past the table's end, inside the lookups
+    return offsets, n
+
+
+@pytest.mark.parametrize("where,n,D", [
+    ("table", 9_000, 64),          # one launch plans and sorts
+    ("table", 200_000, 64),        # counts summed in the scatter
+    ("table", 1_300_000, 8),       # counts scanned
+    ("table", 9_000, 520),         # rows of more than 512 elements
+    ("bag", 200_000, 64), ("bag", 1_300_000, 8), ("bag", 9_000, 520),
+])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_backward_changes_nothing_when_offsets_decrease(where, n, D, weighted):
+    """Offsets that decrease are an error of the caller's: it is flagged, and no row is changed."""
+    rng = workloads.rng_for(487)
+    T, B = 4, 3000
+    lengths = rng.multinomial(n, np.ones(T * B) / (T * B)).astype(np.int64)
+    offsets, n = _disordered(where, T, B, lengths)
+    assert offsets.min() >= 0 and offsets.max() <= n and np.any(np.diff(offsets) < 0)
+    rows = [900, 40, 70_000, 5]     # a key of one table is no row of the next
+    W, wo, Do = helpers.float_tables(rng, rows, [D] * T, np.float32, -0.5, 0.5)
+    hs = np.concatenate([[0], np.cumsum(rows)]).astype(np.int64)
+    indices = rng.integers(0, 5, size=n, dtype=np.int64)
+    dW, dm = _dev(W), torch.full((int(hs[-1]),), 0.25, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    psw = _dev(rng.random(n).astype(np.float32)) if weighted else None
+    cabi.backward(dW, _dev(wo), _dev(Do), _dev(hs), int(hs[-1] - 1).bit_length(), D, _dev(indices), _dev(offsets), B,
+                  torch.ones((B, T * D), device="cuda"), oracle.ROWWISE_ADAGRAD, 0.1, 1e-8, dm, _dev(hs[:-1].copy()),
+                  per_sample_weights=psw, status=status, max_table_rows=max(rows))
+    torch.cuda.synchronize()
+    assert int(status.item()) & cabi.DEV_OFFSETS_NOT_MONOTONE
+    assert np.array_equal(dW.cpu().numpy(), W) and bool((dm == 0.25).all())
+
+
+@pytest.mark.parametrize("n,bits", [(20_000, 7), (20_000, 20), (1_300_000, 7), (1_300_000, 20)])
+def test_segments_that_end_before_they_begin_leave_no_trace_outside(n, bits):
+    """b200tbe_radix_sort_segments with offsets that decrease: nothing is written outside the arrays, and what the
+    input held is still there."""
+    guard = 4096
+    seg = torch.tensor([0, n, n // 4, n, n // 2, n], device="cuda")
+    bufs = [torch.full((n + 2 * guard,), -7, dtype=torch.int32, device="cuda") for _ in range(4)]
+    ki, vi, ko, vo = (b[guard:guard + n] for b in bufs)
+    ki.copy_(torch.randint(0, 1 << bits, (n,), device="cuda", dtype=torch.int32))
+    vi.copy_(torch.arange(n, device="cuda", dtype=torch.int32))
+    before = ki.clone()
+    need = int(cabi.lib().b200tbe_radix_sort_segments_scratch_bytes(n, 5))
+    scratch = torch.zeros(need + 2 * guard, dtype=torch.uint8, device="cuda")
+    st = cabi.lib().b200tbe_radix_sort_segments(ki.data_ptr(), vi.data_ptr(), ko.data_ptr(), vo.data_ptr(), n, seg.data_ptr(), 8,
+                                                5, bits, scratch.data_ptr() + guard, need,
+                                                torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert st == 0 and torch.equal(ki, before)
+    for b in bufs:
+        assert bool((b[:guard] == -7).all()) and bool((b[-guard:] == -7).all())
+    assert int(scratch[:guard].sum()) == 0 and int(scratch[-guard:].sum()) == 0

@@ -19,7 +19,7 @@ MAX_JAGGED_DIMS = 4
 FP32, FP16, INT8, INT4, INT2, BF16 = 0, 1, 2, 3, 4, 5
 POOL_SUM, POOL_MEAN, POOL_NONE = 0, 1, 2
 OPT_SGD, OPT_ROWWISE_ADAGRAD = 0, 1
-DEV_INDEX_OUT_OF_RANGE = 1
+DEV_INDEX_OUT_OF_RANGE, DEV_OFFSETS_NOT_MONOTONE = 1, 2
 
 _c_void_p = ctypes.c_void_p
 

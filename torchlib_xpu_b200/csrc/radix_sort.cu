@@ -80,10 +80,20 @@ __global__ void __launch_bounds__(kSortThreads)
     sort_histogram_kernel(const KeyT* __restrict__ keys, int64_t n, int shift, uint32_t mask,
                           int radix, uint32_t* __restrict__ counts, int num_tiles,
                           const uint4* __restrict__ desc, const uint32_t* __restrict__ seg_tile_base,
-                          const uint32_t* __restrict__ total_tiles) {
+                          const uint32_t* __restrict__ total_tiles, const SortVeto veto) {
   constexpr int kItems = SortTile<KeyT>::kItems;
   constexpr int kTile = SortTile<KeyT>::kTile;
   __shared__ uint32_t hist[kMaxRadix];
+  if (sizeof(KeyT) == 4 && veto.count > 0) {   // this CTA's share of the flags (plans have 4-byte keys)
+    const int64_t each = (veto.count + gridDim.x - 1) / gridDim.x;
+    const int64_t last = (blockIdx.x + 1) * each < veto.count ? (blockIdx.x + 1) * each : veto.count;
+    bool set = false;
+    for (int64_t i = blockIdx.x * each + threadIdx.x; i < last; i += kSortThreads) set = set || __ldg(veto.flags + i) != 0;
+    if (set) {
+      if (veto.status != nullptr) atomicOr(veto.status, B200TBE_DEV_OFFSETS_NOT_MONOTONE);
+      atomicExch(veto.total_tiles, 0u);
+    }
+  }
   const TilePlace tp = place_tile<kTile>(kSum, n, radix, num_tiles, desc, seg_tile_base, total_tiles);
   if (!tp.live) return;
   // all of the thread's keys are requested before the first is counted
@@ -367,11 +377,13 @@ int sort_impl(KeyT* keys_a, uint32_t* vals_a, KeyT* keys_b, uint32_t* vals_b, in
     KeyT* kout = in_b ? keys_a : keys_b;
     uint32_t* vout = in_b ? vals_a : vals_b;
     const PassArgs a{n, shift, bits, tiles, counts, plan};
+    const uint32_t* hist_tiles = plan == nullptr ? nullptr : (pass == 0 ? plan->planned_tiles : plan->total_tiles);
+    const SortVeto veto = plan != nullptr && pass == 0 ? plan->veto : SortVeto{};
     const bool sum = plan != nullptr && bits <= 8 && n / kSortPlanTile <= kSumTiles;
     if constexpr (sizeof(KeyT) == 4) {   // segments have 4-byte keys
       if (sum) {
         sort_histogram_kernel<KeyT, true><<<tiles, kSortThreads, 0, stream>>>(
-            kin, n, shift, mask, radix, counts, tiles, plan->tile_desc, plan->seg_tile_base, plan->total_tiles);
+            kin, n, shift, mask, radix, counts, tiles, plan->tile_desc, plan->seg_tile_base, hist_tiles, veto);
         const int st = launch_scatter_256<KeyT, true>(kin, vin, kout, vout, a, stream);
         if (st != B200TBE_OK) return st;
         in_b = !in_b;
@@ -381,7 +393,7 @@ int sort_impl(KeyT* keys_a, uint32_t* vals_a, KeyT* keys_b, uint32_t* vals_b, in
     }
     sort_histogram_kernel<KeyT, false><<<tiles, kSortThreads, 0, stream>>>(
         kin, n, shift, mask, radix, counts, tiles, plan ? plan->tile_desc : nullptr,
-        plan ? plan->seg_tile_base : nullptr, plan ? plan->total_tiles : nullptr);
+        plan ? plan->seg_tile_base : nullptr, hist_tiles, veto);
     // with a plan the scan also covers the unused tail of the matrix (tiles is an upper bound);
     // nothing reads it
     int st = exclusive_scan_u32(counts, static_cast<int64_t>(radix) * tiles, tile_sums, nullptr, stream);
@@ -445,6 +457,7 @@ SortPlanMem sort_plan_mem(int64_t n, int64_t num_segments, void* plan_mem) {
   m.seg_tile_base = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(num_segments + 1) * 4));
   m.tile_desc = reinterpret_cast<uint4*>(take(static_cast<size_t>(tiles) * sizeof(uint4)));
   m.total_tiles = reinterpret_cast<uint32_t*>(at);
+  m.planned_tiles = m.total_tiles + 1;
   return m;
 }
 

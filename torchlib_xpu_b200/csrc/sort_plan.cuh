@@ -13,6 +13,7 @@ __device__ __forceinline__ void plan_sort(const void* __restrict__ offsets, int 
                                           int32_t* status) {
   const int threads = static_cast<int>(blockDim.x);
   uint32_t carry = 0;
+  bool ordered = true;
   auto start_of = [&](int s) -> int64_t {
     const int64_t i = static_cast<int64_t>(s) * stride;
     int64_t v = offset_bytes == 8 ? load_index<int64_t>(offsets, i) : load_index<int32_t>(offsets, i);
@@ -27,6 +28,7 @@ __device__ __forceinline__ void plan_sort(const void* __restrict__ offsets, int 
       mem.seg_start[s] = static_cast<uint32_t>(first);
       if (s < num_segments) {
         const int64_t len = start_of(s + 1) - first;
+        ordered = ordered && len >= 0;
         tiles = len > 0 ? static_cast<uint32_t>((len + kSortPlanTile - 1) / kSortPlanTile) : 0u;
       }
     }
@@ -35,12 +37,13 @@ __device__ __forceinline__ void plan_sort(const void* __restrict__ offsets, int 
     if (s <= num_segments) mem.seg_tile_base[s] = carry + prefix;
     carry += total;
   }
-  if (carry > static_cast<uint32_t>(max_tiles)) {   // offsets that do not describe n keys
+  // Segments that end before they begin would overlap others: no tile is in use then, so that nothing is sorted
+  // and nothing done with the result. (The barrier: the segments are written.)
+  if (!__syncthreads_and(ordered && carry <= static_cast<uint32_t>(max_tiles))) {
     if (threadIdx.x == 0 && status != nullptr) atomicOr(status, B200TBE_DEV_OFFSETS_NOT_MONOTONE);
-    carry = static_cast<uint32_t>(max_tiles);
+    carry = 0;
   }
-  if (threadIdx.x == 0) *mem.total_tiles = carry;
-  __syncthreads();   // the segments are written
+  if (threadIdx.x == 0) *mem.planned_tiles = *mem.total_tiles = carry;
   for (uint32_t tile = threadIdx.x; tile < carry; tile += threads) {
     // the last segment whose first tile is <= tile (empty segments share their successor's value)
     int lo = 0, hi = num_segments - 1;

@@ -71,7 +71,7 @@ struct BwdDev {
   const uint32_t* sorted_vals;
   uint32_t* bag_of_pos;      // only with per-sample weights
   uint32_t* run_start;       // [num_runs + 1]
-  uint32_t* counters;        // [0] runs, [1] long runs, [2] chunks
+  uint32_t* counters;        // [0] runs, [1] long runs, [2] chunks, [3] offsets decrease somewhere
   uint32_t* long_run;        // [max_long] run id of each long run
   uint32_t* long_chunk0;     // [max_long] first chunk of each long run
   uint32_t* chunk_run;       // [max_chunks] slot (index into long_run) of each chunk
@@ -97,15 +97,22 @@ __global__ void __launch_bounds__(kBwdThreads)
   const int64_t bag0 = (static_cast<int64_t>(blockIdx.x) * kBwdWarps + (threadIdx.x >> 5)) * 32;
   if (bag0 >= total_bags) return;
   const int nb = total_bags - bag0 < 32 ? static_cast<int>(total_bags - bag0) : 32;
-  const int64_t begin = load_index<IndexT>(p.offsets, bag0);
-  const int64_t end = load_index<IndexT>(p.offsets, bag0 + nb);
+  int64_t begin = load_index<IndexT>(p.offsets, bag0);
+  int64_t end = load_index<IndexT>(p.offsets, bag0 + nb);
   const int64_t mine = load_index<IndexT>(p.offsets, bag0 + (lane < nb ? lane : nb));
+  const int64_t after = __shfl_down_sync(kFullMask, mine, 1);
+  if (mine > (lane == 31 ? end : after)) {   // positions without a key: write_run_starts_kernel then leaves no runs
+    if (p.status != nullptr) atomicOr(p.status, B200TBE_DEV_OFFSETS_NOT_MONOTONE);
+    atomicOr(p.counters + 3, 1u);
+  }
+  if (begin < 0) begin = 0;
+  if (end > p.num_indices) end = p.num_indices;
   // a group of 32 bags longer than 2^32 lookups does not occur in memory that exists
   const uint32_t my_start = static_cast<uint32_t>(mine - begin);
   const int my_t = static_cast<int>((bag0 + (lane < nb ? lane : nb - 1)) / p.B);
   const int64_t my_h0 = __ldg(p.hash_size_cumsum + my_t);
   const int64_t my_rows = __ldg(p.hash_size_cumsum + my_t + 1) - my_h0;
-  const uint32_t total = static_cast<uint32_t>(end - begin);
+  const uint32_t total = end > begin ? static_cast<uint32_t>(end - begin) : 0u;
   for (uint32_t base = 0; base < total; base += 32) {
     const uint32_t rel = base + lane;
     // the last bag whose start is <= rel (empty bags share a start with their successor)
@@ -159,7 +166,7 @@ template <typename KeyT>
 __global__ void __launch_bounds__(kSegThreads)
     write_run_starts_kernel(const KeyT* __restrict__ keys, int64_t n,
                             const uint32_t* __restrict__ tile_heads,
-                            const uint32_t* __restrict__ counters, uint32_t* __restrict__ run_start) {
+                            uint32_t* counters, uint32_t* __restrict__ run_start) {
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kSegTile + threadIdx.x * kSegItems;
   bool head[kSegItems];
   uint32_t c = 0;
@@ -173,7 +180,10 @@ __global__ void __launch_bounds__(kSegThreads)
 #pragma unroll
   for (int i = 0; i < kSegItems; ++i)
     if (head[i]) run_start[at++] = static_cast<uint32_t>(base + i);
-  if (blockIdx.x == 0 && threadIdx.x == 0) run_start[counters[0]] = static_cast<uint32_t>(n);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    run_start[counters[0]] = static_cast<uint32_t>(n);
+    if (counters[3] != 0) counters[0] = 0;
+  }
 }
 
 __device__ __forceinline__ int64_t bag_length(const BwdDev& p, int64_t bag) {
@@ -991,16 +1001,23 @@ int run_backward_sweep(BwdDev d, const b200tbe_backward_params* p, const Scratch
     d.sorted_keys = s.keys[result];
     d.sorted_vals = s.vals[result];
   } else {
-    const SortPlan plan = sort_plan_of(mem, max_tiles);
+    SortPlan plan = sort_plan_of(mem, max_tiles);
     const int64_t bags = static_cast<int64_t>(p->T) * p->B;
     const int64_t lin_ctas = 1 + (bags + 32 * kBwdWarps - 1) / (32 * kBwdWarps);
     if (lin_ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
+    // one flag per group of 32 bags, in memory that the sort does not use before it has read them
+    uint8_t* flags = reinterpret_cast<uint8_t*>(vals_b);
+    const int64_t groups = (bags + 31) / 32, num_flags = groups < 4 * n ? groups : 4 * n;
+    const bool all_flags = groups == num_flags;
+    if (!all_flags && cudaMemsetAsync(flags, 0, static_cast<size_t>(num_flags), stream) != cudaSuccess)
+      return B200TBE_ERR_LAUNCH;
+    plan.veto = SortVeto{flags, num_flags, mem.total_tiles, p->status};
     if (weighted) {
-      linearize_rows_kernel<IndexT, true>
-          <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a, mem, max_tiles);
+      linearize_rows_kernel<IndexT, true><<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(
+          d, key_bits, keys_a, vals_a, mem, max_tiles, flags, num_flags, all_flags);
     } else {
-      linearize_rows_kernel<IndexT, false>
-          <<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(d, key_bits, keys_a, vals_a, mem, max_tiles);
+      linearize_rows_kernel<IndexT, false><<<static_cast<unsigned>(lin_ctas), kBwdThreads, 0, stream>>>(
+          d, key_bits, keys_a, vals_a, mem, max_tiles, flags, num_flags, all_flags);
     }
     bool in_b = false;
     const int st = radix_sort_pairs_planned(keys_a, vals_a, keys_b, vals_b, n, key_bits, kSweepSortDigitBits, plan,

@@ -62,10 +62,13 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallTh
   // ---- the plan: this table's tiles follow those of the tables before it ----
   if (rank_in_cluster == 0) {
     uint32_t before = 0;
+    bool ordered = seg_begin <= seg_next;
     for (int q = threadIdx.x; q < t; q += kSmallThreads) {
       const uint32_t a = start_of(q), b = start_of(q + 1);
       before += b > a ? (b - a + kSortPlanTile - 1) / kSortPlanTile : 0u;
+      ordered = ordered && a <= b;
     }
+    const bool good = __syncthreads_and(ordered);   // of the tables up to this one: the last table's CTA sees all
     uint32_t first;
     block_exclusive_scan(before, &first);
     const uint32_t tiles = (seg_len + kSortPlanTile - 1) / kSortPlanTile;
@@ -79,12 +82,9 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallTh
       s.seg_start[t] = seg_begin;
       if (t == p.T - 1) {
         s.seg_start[p.T] = seg_next;
-        uint32_t total = first + tiles;
-        if (total > static_cast<uint32_t>(s.max_tiles)) {   // offsets that do not describe n lookups
-          if (p.status != nullptr) atomicOr(p.status, B200TBE_DEV_OFFSETS_NOT_MONOTONE);
-          total = static_cast<uint32_t>(s.max_tiles);
-        }
-        *s.total_tiles = total;
+        // tables that end before they begin would overlap others: nothing is done with what is sorted
+        if (!good && p.status != nullptr) atomicOr(p.status, B200TBE_DEV_OFFSETS_NOT_MONOTONE);
+        *s.total_tiles = good ? first + tiles : 0u;
       }
     }
   }

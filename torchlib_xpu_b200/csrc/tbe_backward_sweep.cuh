@@ -116,10 +116,13 @@ __device__ __forceinline__ float sqrt_fast(float x) {
 // ---- linearize with per-table keys -------------------------------------------------------------
 // As linearize_kernel, but the key is the row id alone: the table is implied by the position. The first CTA
 // builds the sort's plan meanwhile, which needs two launches (9 us) less than a launch before this one.
+// A warp whose offsets decrease leaves a flag: positions may then have a key of another table or none at all.
+// flags has a place for every warp (all_flags), or holds zeros and only the flags that are set are written.
 template <typename IndexT, bool kWeighted>
 __global__ void __launch_bounds__(kBwdThreads)
     linearize_rows_kernel(BwdDev p, int key_bits, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                          const SortPlanMem plan, int max_tiles) {
+                          const SortPlanMem plan, int max_tiles, uint8_t* __restrict__ flags, int64_t num_flags,
+                          bool all_flags) {
   if (blockIdx.x == 0) {
     plan_sort(p.offsets, static_cast<int>(sizeof(IndexT)), p.T, p.B, p.num_indices, max_tiles, plan, p.status);
     return;
@@ -129,10 +132,14 @@ __global__ void __launch_bounds__(kBwdThreads)
   const int64_t bag0 = (static_cast<int64_t>(blockIdx.x - 1) * kBwdWarps + (threadIdx.x >> 5)) * 32;
   if (bag0 >= total_bags) return;
   const int nb = total_bags - bag0 < 32 ? static_cast<int>(total_bags - bag0) : 32;
-  const int64_t begin = load_index<IndexT>(p.offsets, bag0);
+  int64_t begin = load_index<IndexT>(p.offsets, bag0);
   int64_t end = load_index<IndexT>(p.offsets, bag0 + nb);
-  if (end > p.num_indices) end = p.num_indices;
   const int64_t mine = load_index<IndexT>(p.offsets, bag0 + (lane < nb ? lane : nb));
+  const int64_t after = __shfl_down_sync(kFullMask, mine, 1);
+  const bool disordered = __any_sync(kFullMask, mine > (lane == 31 ? end : after));
+  if (lane == 0 && (all_flags || disordered)) flags[(bag0 >> 5) % num_flags] = disordered;
+  if (begin < 0) begin = 0;
+  if (end > p.num_indices) end = p.num_indices;
   const uint32_t my_start = static_cast<uint32_t>(mine - begin);
   const int my_t = static_cast<int>((bag0 + (lane < nb ? lane : nb - 1)) / p.B);
   int64_t my_rows = __ldg(p.hash_size_cumsum + my_t + 1) - __ldg(p.hash_size_cumsum + my_t);
