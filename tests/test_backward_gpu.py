@@ -501,3 +501,39 @@ def test_segments_that_end_before_they_begin_leave_no_trace_outside(n, bits):
     for b in bufs:
         assert bool((b[:guard] == -7).all()) and bool((b[-guard:] == -7).all())
     assert int(scratch[:guard].sum()) == 0 and int(scratch[-guard:].sum()) == 0
+
+
+@pytest.mark.parametrize("n", [5000, 200_000, 1_300_000])
+def test_backward_offsets_that_begin_after_the_first_lookup(n):
+    """Lookups before offsets[0] belong to no bag (a slice of a longer batch's offsets): every sort leaves them out."""
+    rng = workloads.rng_for(488)
+    rows, Ds, B, skip = [300, 2000], [8, 16], 900, 4099
+    lengths = rng.multinomial(n, np.ones(2 * B) / (2 * B)).astype(np.int64)
+    offsets = np.zeros(2 * B + 1, dtype=np.int64)
+    np.cumsum(lengths, out=offsets[1:])
+    indices = np.concatenate([rng.integers(0, rows[t], size=int(offsets[(t + 1) * B] - offsets[t * B])) for t in range(2)])
+    W, wo, Do = helpers.float_tables(rng, rows, Ds, np.float32, -0.5, 0.5)
+    hs = np.concatenate([[0], np.cumsum(rows)]).astype(np.int64)
+    grad = rng.integers(-8, 9, size=(B, sum(Ds))).astype(np.float32) / 64
+    W_ref = W.copy()
+    oracle.tbe_backward(W_ref, oracle.FP32, wo, Do, hs, B, indices, offsets, grad, None, None, oracle.SGD, 0.5, 0.0, None)
+    dW = _dev(W)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    longer = np.concatenate([rng.integers(0, 300, size=skip), indices])
+    cabi.backward(dW, _dev(wo), _dev(Do), _dev(hs), 12, 16, _dev(longer), _dev(offsets + skip), B, _dev(grad), oracle.SGD,
+                  0.5, status=status, max_table_rows=max(rows))
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    np.testing.assert_allclose(dW.cpu().numpy(), W_ref, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("bits", [8, 19])
+def test_segmented_sort_of_segments_that_begin_after_the_first_key(bits):
+    rng = workloads.rng_for(489)
+    n, seg = 1_300_000, np.array([5001, 5001, 700_000, 1_300_000])
+    keys, vals = rng.integers(0, 1 << bits, size=n, dtype=np.int32), np.arange(n, dtype=np.int32)
+    ks, vs = cabi.radix_sort_segments(_dev(keys), _dev(vals), _dev(seg), bits)
+    ks, vs = ks.cpu().numpy(), vs.cpu().numpy()
+    for a, b in zip(seg[:-1], seg[1:]):
+        order = np.argsort(keys[a:b], kind="stable")
+        assert np.array_equal(ks[a:b], keys[a:b][order]) and np.array_equal(vs[a:b], vals[a:b][order])

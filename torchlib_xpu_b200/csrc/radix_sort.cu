@@ -394,9 +394,9 @@ int sort_impl(KeyT* keys_a, uint32_t* vals_a, KeyT* keys_b, uint32_t* vals_b, in
     sort_histogram_kernel<KeyT, false><<<tiles, kSortThreads, 0, stream>>>(
         kin, n, shift, mask, radix, counts, tiles, plan ? plan->tile_desc : nullptr,
         plan ? plan->seg_tile_base : nullptr, hist_tiles, veto);
-    // with a plan the scan also covers the unused tail of the matrix (tiles is an upper bound);
+    // with a plan the scan starts where the first segment does, and also covers the unused tail of the matrix (tiles is an upper bound);
     // nothing reads it
-    int st = exclusive_scan_u32(counts, static_cast<int64_t>(radix) * tiles, tile_sums, nullptr, stream);
+    int st = exclusive_scan_u32(counts, static_cast<int64_t>(radix) * tiles, tile_sums, plan ? plan->seg_start : nullptr, stream);
     if (st != B200TBE_OK) return st;
     if (bits <= 8) {
       st = launch_scatter_256<KeyT, false>(kin, vin, kout, vout, a, stream);

@@ -34,6 +34,7 @@ struct SortVeto {
 };
 
 struct SortPlan {
+  const uint32_t* seg_start;       // [segments + 1] first key of each segment
   const uint4* tile_desc;          // [max_tiles] {first key, key count, segment, first tile of the segment}
   const uint32_t* seg_tile_base;   // [segments + 1] exclusive prefix of the tiles per segment
   const uint32_t* planned_tiles;   // device scalar: tiles of the plan (<= max_tiles), for the first histogram
@@ -58,7 +59,7 @@ struct SortPlanMem {
 };
 SortPlanMem sort_plan_mem(int64_t n, int64_t num_segments, void* plan_mem);
 inline SortPlan sort_plan_of(const SortPlanMem& m, int max_tiles) {
-  return SortPlan{m.tile_desc, m.seg_tile_base, m.planned_tiles, m.total_tiles, max_tiles, SortVeto{}};
+  return SortPlan{m.seg_start, m.tile_desc, m.seg_tile_base, m.planned_tiles, m.total_tiles, max_tiles, SortVeto{}};
 }
 bool sort_plan_fits(int64_t max_tiles);   // the sort's counts of so many tiles are numbered in 31 bits
 

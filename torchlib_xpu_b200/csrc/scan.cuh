@@ -58,11 +58,12 @@ static __global__ void __launch_bounds__(kScanThreads)
   if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-// In-place exclusive scan of `count` values by a single CTA; the grand total goes to *total_out
-// when that is not null.
+// In-place exclusive scan of `count` values by a single CTA, from *first on (null: from 0); the grand total goes
+// to *total_out when that is not null.
 static __global__ void __launch_bounds__(kScanThreads)
-    scan_single_cta_kernel(uint32_t* __restrict__ vals, int64_t count, uint32_t* total_out) {
-  uint32_t carry = 0;
+    scan_single_cta_kernel(uint32_t* __restrict__ vals, int64_t count, uint32_t* total_out,
+                           const uint32_t* __restrict__ first = nullptr) {
+  uint32_t carry = first != nullptr ? *first : 0u;
   for (int64_t base = 0; base < count; base += kScanThreads) {
     const int64_t i = base + threadIdx.x;
     const uint32_t v = i < count ? vals[i] : 0;
@@ -94,14 +95,15 @@ static __global__ void __launch_bounds__(kScanThreads)
   }
 }
 
-// data[0..n) <- exclusive prefix sums, in place. tile_sums needs scan_num_tiles(n) entries.
-inline int exclusive_scan_u32(uint32_t* data, int64_t n, uint32_t* tile_sums, uint32_t* total_out,
+// data[0..n) <- exclusive prefix sums from *first on (null: from 0), in place. tile_sums needs scan_num_tiles(n)
+// entries.
+inline int exclusive_scan_u32(uint32_t* data, int64_t n, uint32_t* tile_sums, const uint32_t* first,
                               cudaStream_t stream) {
   if (n <= 0) return B200TBE_OK;
   const int64_t tiles = scan_num_tiles(n);
   if (tiles > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
   scan_tile_sums_kernel<<<static_cast<unsigned>(tiles), kScanThreads, 0, stream>>>(data, n, tile_sums);
-  scan_single_cta_kernel<<<1, kScanThreads, 0, stream>>>(tile_sums, tiles, total_out);
+  scan_single_cta_kernel<<<1, kScanThreads, 0, stream>>>(tile_sums, tiles, nullptr, first);
   scan_apply_kernel<<<static_cast<unsigned>(tiles), kScanThreads, 0, stream>>>(data, n, tile_sums);
   return launch_status();
 }
