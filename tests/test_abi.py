@@ -52,3 +52,20 @@ def test_argument_validation_needs_no_gpu():
     assert lib.b200tbe_radix_sort_pairs(None, None, None, None, -1, 4, 8, None, 0, None) == -1
     assert lib.b200tbe_radix_sort_scratch_bytes(0) >= 0
     assert lib.b200tbe_backward_scratch_bytes(1 << 20, 25, 128, 8) > (1 << 20) * 8
+
+
+def test_permute_rows_refuses_widths_it_does_not_move():
+    """Before anything is launched: no width, and no pair of widths, is taken for another. (The pointers are never
+    followed on the host.)"""
+    lib = cabi.lib()
+    at = ctypes.c_void_p(1 << 20)
+    call = lambda e, e2, second: lib.b200tbe_permute_rows(  # noqa: E731
+        at, at, e, at if second else None, at if second else None, e2, at, at, ctypes.c_int64(1), ctypes.c_int64(1), None)
+    for width in (0, 1, 3, 6, 7, 16, -4):
+        assert call(width, 0, False) == -4
+        assert call(width, 4, True) == -4
+        assert call(4, width, True) == -4
+    for e, e2 in ((4, 64), (2, 32), (1, 16), (7, 16), (3, 20), (2, 96), (4, 0)):
+        assert call(e, e2, True) == -4
+    # nothing to move: any widths, as ever
+    assert lib.b200tbe_permute_rows(None, None, 3, None, None, 0, None, None, ctypes.c_int64(0), ctypes.c_int64(1), None) == 0

@@ -424,6 +424,8 @@ extern "C" int b200tbe_permute_rows(const void* in, void* out, int32_t elem_byte
   if (out_rows == 0 || total_elems == 0) return B200TBE_OK;
   if (in == nullptr || out == nullptr || in_start == nullptr || out_offsets == nullptr || (in2 == nullptr) != (out2 == nullptr))
     return B200TBE_ERR_BAD_ARG;
+  auto moved = [](int bytes) { return bytes == 2 || bytes == 4 || bytes == 8; };
+  if (!moved(elem_bytes) || (in2 != nullptr && !moved(elem2_bytes))) return B200TBE_ERR_UNSUPPORTED;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const int second = in2 != nullptr ? elem2_bytes : 0;
   switch (elem_bytes * 16 + second) {
@@ -434,7 +436,6 @@ extern "C" int b200tbe_permute_rows(const void* in, void* out, int32_t elem_byte
     case 4 * 16 + 4: return move_rows<uint32_t, uint32_t>(in, out, in2, out2, in_start, out_offsets, out_rows, total_elems, stream);
     default: break;
   }
-  if (second == 0) return B200TBE_ERR_UNSUPPORTED;
   // any other pair of widths: one array after the other
   const int st = b200tbe_permute_rows(in, out, elem_bytes, nullptr, nullptr, 0, in_start, out_offsets, out_rows, total_elems, stream_);
   if (st != B200TBE_OK) return st;
