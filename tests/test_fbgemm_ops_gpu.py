@@ -229,3 +229,30 @@ def test_permute_2d_sparse_data_shapes_and_types(T, B, hi, P, id_dtype, w_dtype,
         pl, pi, pw = torch.ops.fbgemm.permute_2D_sparse_data(cuda(permute), cuda(lengths), cuda(indices), cuda(weights), given)
         assert torch.equal(pl.cpu(), lengths[permute.long()]) and torch.equal(pi.cpu(), indices[at])
         assert pw is None if weights is None else torch.equal(pw.cpu(), weights[at])
+
+
+@pytest.mark.parametrize("T,B,hi,P", [
+    (1, 700_000, 1, 1), (3, 140_000, 2, 5),              # rows of many chunks, summed by a warp
+    (1025, 3, 4, 1025), (4097, 2, 3, 4095),              # one to two tiles of rows in one CTA
+    (8192, 1, 3, 8192), (8193, 1, 3, 8192), (8191, 4, 2, 8193), (5, 40, 6, 30_000), (30_000, 3, 2, 7),   # and beyond
+    (300, 511, 2, 300), (300, 512, 2, 300), (300, 513, 2, 300),   # either side of the short rows' kernel
+    (9000, 5000, 0, 9000),                               # many rows of two chunks
+])
+@pytest.mark.parametrize("len_dtype,perm_dtype", [(torch.int32, torch.int64), (torch.int64, torch.int32)])
+def test_permute_2d_sparse_data_long_rows_and_many_rows(T, B, hi, P, len_dtype, perm_dtype):
+    gen = torch.Generator(device="cuda").manual_seed(T + B)
+    lengths = torch.randint(0, hi + 1, (T, B), device="cuda", generator=gen).to(len_dtype)
+    if hi == 0:
+        lengths[::7, ::41] = 3
+    rows = lengths.long().sum(1)
+    total = int(rows.sum())
+    ids = torch.arange(total, device="cuda")
+    permute = torch.randint(0, T, (P,), device="cuda", generator=gen).to(perm_dtype)
+    start = torch.cumsum(rows, 0) - rows
+    out_len = rows[permute.long()]
+    out_start = torch.cumsum(out_len, 0) - out_len
+    count = int(out_len.sum())
+    at = torch.arange(count, device="cuda") + torch.repeat_interleave(start[permute.long()] - out_start, out_len, output_size=count)
+    for given in (None, count):
+        pl, pi, _ = torch.ops.fbgemm.permute_2D_sparse_data(permute, lengths, ids, None, given)
+        assert torch.equal(pl, lengths[permute.long()]) and torch.equal(pi, at)

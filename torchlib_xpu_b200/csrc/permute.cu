@@ -273,7 +273,37 @@ __global__ void __launch_bounds__(kLenThreads)
   }
 }
 
+// Short rows: a group of 2^shift lanes, as many as the row has columns (32 at most), takes one. (With a CTA per row
+// and one CTA finding all places, below, a call over 20 000 / 100 000 / 1 000 000 rows took 152 / 721 / 7096 us; 52 /
+// 54 / 103 now.)
+constexpr int kShortCols = 512;
+
+template <typename LenT, typename PermT>
+__global__ void __launch_bounds__(kLenThreads)
+    permute_short_lengths_kernel(const LenT* __restrict__ lengths, const PermT* __restrict__ perm,
+                                 LenT* __restrict__ permuted, int64_t* __restrict__ row_sums, int64_t rows, int cols,
+                                 int64_t out_rows, int shift) {
+  const int64_t y = (static_cast<int64_t>(blockIdx.x) * kLenThreads + threadIdx.x) >> shift;
+  const int g = 1 << shift, lane = threadIdx.x & (g - 1);
+  int64_t sum = 0;
+  if (y < rows) {
+    const LenT* src = lengths + y * cols;
+#pragma unroll 4
+    for (int c = lane; c < cols; c += g) sum += static_cast<int64_t>(src[c]);
+  } else if (y < rows + out_rows) {
+    const int64_t from = static_cast<int64_t>(perm[y - rows]);
+    assert(from >= 0 && from < rows);
+    const LenT* src = lengths + from * cols;
+    LenT* dst = permuted + (y - rows) * cols;
+#pragma unroll 4
+    for (int c = lane; c < cols; c += g) dst[c] = src[c];
+  }
+  for (int o = g >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
+  if (y < rows && lane == 0) row_sums[y] = sum;
+}
+
 constexpr int kRowThreads = 1024;
+constexpr int kRowTile = kRowThreads * 4;   // rows of a tile, where there are more rows than threads
 
 // Exclusive sum over the CTA's threads; *total is the CTA's sum.
 __device__ __forceinline__ int64_t exclusive_sum(int64_t v, int64_t* total) {
@@ -299,58 +329,190 @@ __device__ __forceinline__ int64_t exclusive_sum(int64_t v, int64_t* total) {
   return before + incl - v;
 }
 
-// One CTA: where every input row starts, then where every output row starts and where it comes from.
+// The lengths of input rows, and of output rows with where they come from.
+struct InputRows {
+  const int64_t* __restrict__ chunk_sums;
+  int64_t chunks;
+  __device__ __forceinline__ int64_t length(int64_t r, int64_t*) const {
+    int64_t len = 0;
+#pragma unroll 4
+    for (int64_t k = 0; k < chunks; ++k) len += chunk_sums[r * chunks + k];
+    return len;
+  }
+};
+struct SummedRows {
+  const int64_t* sums;   // (written earlier in the same launch)
+  __device__ __forceinline__ int64_t length(int64_t r, int64_t*) const { return sums[r]; }
+};
 template <typename PermT>
+struct OutputRows {
+  const PermT* __restrict__ perm;
+  const int64_t* in_offsets;   // (written earlier in the same launch, where one CTA does it all)
+  int64_t rows;
+  __device__ __forceinline__ int64_t length(int64_t j, int64_t* start) const {
+    const int64_t from = static_cast<int64_t>(perm[j]);
+    if (from < 0 || from >= rows) {
+      *start = 0;
+      return 0;
+    }
+    *start = in_offsets[from];
+    return in_offsets[from + 1] - *start;
+  }
+};
+
+// offsets[i], i in the tile [base, base + kRowThreads * kItems) of n rows = carry + the lengths of the tile's rows
+// before i; starts, where given, receives the rows' starts. Returns the tile's sum.
+template <int kItems, typename Rows>
+__device__ __forceinline__ int64_t tile_offsets(const Rows& r, int64_t base, int64_t n, int64_t carry,
+                                                int64_t* offsets, int64_t* __restrict__ starts) {
+  const int64_t i0 = base + static_cast<int64_t>(threadIdx.x) * kItems;
+  int64_t len[kItems], start[kItems], mine = 0;
+#pragma unroll
+  for (int k = 0; k < kItems; ++k) {
+    len[k] = start[k] = 0;
+    if (i0 + k < n) len[k] = r.length(i0 + k, &start[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < kItems; ++k) mine += len[k];
+  int64_t total;
+  int64_t at = carry + exclusive_sum(mine, &total);
+#pragma unroll
+  for (int k = 0; k < kItems; ++k) {
+    if (i0 + k < n) {
+      offsets[i0 + k] = at;
+      if (starts != nullptr) starts[i0 + k] = start[k];
+    }
+    at += len[k];
+  }
+  return total;
+}
+
+// One CTA: where every input row starts, then where every output row starts and where it comes from. Rows of
+// many chunks are summed first, a warp per row (one row of 16 M lengths: the whole call 322 us with a thread per
+// row, 119 so).
+constexpr int64_t kManyChunks = 32;
+
+template <typename PermT, int kItems>
 __global__ void __launch_bounds__(kRowThreads)
     permute_row_starts_kernel(const int64_t* __restrict__ chunk_sums, const PermT* __restrict__ perm,
                               int64_t* in_offsets, int64_t* __restrict__ in_start, int64_t* __restrict__ out_offsets,
                               int64_t rows, int64_t chunks, int64_t out_rows) {
-  int64_t carry = 0, total;
-  for (int64_t base = 0; base < rows; base += kRowThreads) {
-    const int64_t r = base + threadIdx.x;
-    int64_t len = 0;
-    if (r < rows)
-      for (int64_t k = 0; k < chunks; ++k) len += chunk_sums[r * chunks + k];
-    const int64_t before = exclusive_sum(len, &total);
-    if (r < rows) in_offsets[r] = carry + before;
-    carry += total;
+  const bool many = chunks >= kManyChunks;
+  if (many) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t r = threadIdx.x >> 5; r < rows; r += kRowThreads / 32) {
+      int64_t sum = 0;
+#pragma unroll 4
+      for (int64_t k = lane; k < chunks; k += 32) sum += chunk_sums[r * chunks + k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
+      if (lane == 0) in_offsets[r] = sum;   // a row's sum stays there until its offset takes the place
+    }
+    __syncthreads();
   }
+  int64_t carry = 0;
+  for (int64_t base = 0; base < rows; base += kRowThreads * kItems)
+    carry += many ? tile_offsets<kItems>(SummedRows{in_offsets}, base, rows, carry, in_offsets, nullptr)
+                  : tile_offsets<kItems>(InputRows{chunk_sums, chunks}, base, rows, carry, in_offsets, nullptr);
   if (threadIdx.x == 0) in_offsets[rows] = carry;
   __syncthreads();
+  const OutputRows<PermT> out{perm, in_offsets, rows};
   carry = 0;
-  for (int64_t base = 0; base < out_rows; base += kRowThreads) {
-    const int64_t j = base + threadIdx.x;
-    int64_t len = 0, start = 0;
-    if (j < out_rows) {
-      const int64_t from = static_cast<int64_t>(perm[j]);
-      if (from >= 0 && from < rows) {   // (anything else has ended in the lengths kernel)
-        start = in_offsets[from];
-        len = in_offsets[from + 1] - start;
-      }
-      in_start[j] = start;
-    }
-    const int64_t before = exclusive_sum(len, &total);
-    if (j < out_rows) out_offsets[j] = carry + before;
-    carry += total;
-  }
+  for (int64_t base = 0; base < out_rows; base += kRowThreads * kItems)
+    carry += tile_offsets<kItems>(out, base, out_rows, carry, out_offsets, in_start);
   if (threadIdx.x == 0) out_offsets[out_rows] = carry;
 }
+
+// The same for many rows, a CTA per tile: the tiles' sums (kept in the offset of the tile's first row), their
+// prefixes by one CTA, then the offsets.
+template <typename Rows>
+__global__ void __launch_bounds__(kRowThreads) row_tile_sums_kernel(const Rows r, int64_t n, int64_t* offsets) {
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kRowTile;
+  int64_t sum = 0, unused;
+#pragma unroll
+  for (int k = 0; k < kRowTile / kRowThreads; ++k) {
+    const int64_t i = base + k * kRowThreads + threadIdx.x;
+    if (i < n) sum += r.length(i, &unused);
+  }
+  int64_t total;
+  exclusive_sum(sum, &total);
+  if (threadIdx.x == 0) offsets[base] = total;
+}
+
+__global__ void __launch_bounds__(kRowThreads) row_tile_prefixes_kernel(int64_t n, int64_t* offsets) {
+  int64_t carry = 0;
+  for (int64_t base = 0; base < n; base += int64_t{kRowTile} * kRowThreads) {
+    const int64_t i = base + int64_t{kRowTile} * threadIdx.x;
+    const int64_t sum = i < n ? offsets[i] : 0;
+    int64_t total;
+    const int64_t before = exclusive_sum(sum, &total);
+    if (i < n) offsets[i] = carry + before;
+    carry += total;
+  }
+  if (threadIdx.x == 0) offsets[n] = carry;
+}
+
+template <typename Rows>
+__global__ void __launch_bounds__(kRowThreads)
+    row_offsets_kernel(const Rows r, int64_t n, int64_t* offsets, int64_t* __restrict__ starts) {
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kRowTile;
+  const int64_t carry = offsets[base];
+  __syncthreads();   // every thread has it
+  tile_offsets<kRowTile / kRowThreads>(r, base, n, carry, offsets, starts);
+}
+
+template <typename Rows>
+int launch_row_offsets(const Rows& r, int64_t n, int64_t* offsets, int64_t* starts, cudaStream_t stream) {
+  const int64_t tiles = (n + kRowTile - 1) / kRowTile;
+  if (tiles > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
+  if (tiles > 0) row_tile_sums_kernel<Rows><<<static_cast<unsigned>(tiles), kRowThreads, 0, stream>>>(r, n, offsets);
+  row_tile_prefixes_kernel<<<1, kRowThreads, 0, stream>>>(n, offsets);
+  if (tiles > 0) row_offsets_kernel<Rows><<<static_cast<unsigned>(tiles), kRowThreads, 0, stream>>>(r, n, offsets, starts);
+  return launch_status();
+}
+
+// Up to this many rows one CTA does it all: 4096 rows of 64 lengths 50 -> 34 us a call with four rows per thread;
+// the six launches of the other way cost more than that below, and less above.
+constexpr int64_t kOneCtaRows = 2 * kRowTile;
 
 int64_t length_chunks(int64_t cols) { return cols > 0 ? (cols + kLenChunk - 1) / kLenChunk : 1; }
 
 template <typename LenT, typename PermT>
-int launch_row_starts(const void* lengths, const void* perm, void* permuted, int64_t* in_start, int64_t* out_offsets,
+int launch_row_starts(const void* lengths_, const void* perm_, void* permuted_, int64_t* in_start, int64_t* out_offsets,
                       int64_t rows, int64_t cols, int64_t out_rows, int64_t* scratch, cudaStream_t stream) {
+  const LenT* lengths = static_cast<const LenT*>(lengths_);
+  const PermT* perm = static_cast<const PermT*>(perm_);
+  LenT* permuted = static_cast<LenT*>(permuted_);
   const int64_t chunks = length_chunks(cols);
-  const int64_t ctas = (rows + (permuted != nullptr ? out_rows : 0)) * chunks;
-  if (ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
+  const int64_t copied = permuted != nullptr ? out_rows : 0;
+  int64_t* in_offsets = scratch;
   int64_t* chunk_sums = scratch + rows + 1;
-  permute_lengths_kernel<LenT, PermT><<<static_cast<unsigned>(ctas), kLenThreads, 0, stream>>>(
-      static_cast<const LenT*>(lengths), static_cast<const PermT*>(perm), static_cast<LenT*>(permuted), chunk_sums, rows,
-      cols, chunks);
-  permute_row_starts_kernel<PermT><<<1, kRowThreads, 0, stream>>>(chunk_sums, static_cast<const PermT*>(perm), scratch,
-                                                                  in_start, out_offsets, rows, chunks, out_rows);
-  return launch_status();
+  if (cols <= kShortCols) {
+    int shift = 0;
+    while (shift < 5 && (1 << shift) < cols) ++shift;
+    const int64_t ctas = (((rows + copied) << shift) + kLenThreads - 1) / kLenThreads;
+    if (ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
+    permute_short_lengths_kernel<LenT, PermT><<<static_cast<unsigned>(ctas), kLenThreads, 0, stream>>>(
+        lengths, perm, permuted, chunk_sums, rows, static_cast<int>(cols), copied, shift);
+  } else {
+    const int64_t ctas = (rows + copied) * chunks;
+    if (ctas > 0x7fffffff) return B200TBE_ERR_TOO_LARGE;
+    permute_lengths_kernel<LenT, PermT><<<static_cast<unsigned>(ctas), kLenThreads, 0, stream>>>(
+        lengths, perm, permuted, chunk_sums, rows, cols, chunks);
+  }
+  if (rows <= kRowThreads && out_rows <= kRowThreads) {
+    permute_row_starts_kernel<PermT, 1><<<1, kRowThreads, 0, stream>>>(chunk_sums, perm, in_offsets, in_start,
+                                                                       out_offsets, rows, chunks, out_rows);
+    return launch_status();
+  }
+  if (rows <= kOneCtaRows && out_rows <= kOneCtaRows) {
+    permute_row_starts_kernel<PermT, 4><<<1, kRowThreads, 0, stream>>>(chunk_sums, perm, in_offsets, in_start,
+                                                                       out_offsets, rows, chunks, out_rows);
+    return launch_status();
+  }
+  const int st = launch_row_offsets(InputRows{chunk_sums, chunks}, rows, in_offsets, nullptr, stream);
+  if (st != B200TBE_OK) return st;
+  return launch_row_offsets(OutputRows<PermT>{perm, in_offsets, rows}, out_rows, out_offsets, in_start, stream);
 }
 
 }  // namespace
