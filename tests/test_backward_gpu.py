@@ -537,3 +537,29 @@ def test_segmented_sort_of_segments_that_begin_after_the_first_key(bits):
     for a, b in zip(seg[:-1], seg[1:]):
         order = np.argsort(keys[a:b], kind="stable")
         assert np.array_equal(ks[a:b], keys[a:b][order]) and np.array_equal(vs[a:b], vals[a:b][order])
+
+
+@pytest.mark.parametrize("segments,n", [(1023, 60_000), (1024, 60_000), (1025, 2_000_000), (4096, 90_000), (4097, 90_000),
+                                        (20_000, 300_000)])
+def test_segmented_sort_of_many_segments(segments, n):
+    """The plan takes segments by batches of four per thread: either side of a batch, empty segments and segments of
+    several tiles among them, some at a batch's end."""
+    rng = workloads.rng_for(490 + segments)
+    sizes = rng.integers(0, 2, size=segments)
+    for s in (0, 1, segments - 1, segments // 2, min(4095, segments - 1), min(4096, segments - 1)):
+        sizes[s] = 9000
+    sizes[rng.integers(0, segments)] += max(0, n - sizes.sum())
+    seg = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = int(seg[-1])
+    keys, vals = rng.integers(0, 1 << 9, size=n, dtype=np.int32), np.arange(n, dtype=np.int32)
+    ks, vs = cabi.radix_sort_segments(_dev(keys), _dev(vals), _dev(seg), 9)
+    order = np.lexsort((keys, np.repeat(np.arange(segments), sizes)))
+    assert np.array_equal(ks.cpu().numpy(), keys[order]) and np.array_equal(vs.cpu().numpy(), vals[order])
+
+
+@pytest.mark.parametrize("T,B", [(255, 40), (256, 40), (1024, 9), (1025, 9), (2100, 5)])
+def test_backward_over_many_tables(T, B):
+    rng = workloads.rng_for(491 + T)
+    rows, Ds = [60] * T, [8] * T
+    case = _backward_case(rng, rows, Ds, B, 0, 14, np.float32, np.float32, oracle.SUM, oracle.SGD, False)
+    _check(*case, B, np.float32, np.float32, oracle.SUM, oracle.SGD)

@@ -64,7 +64,7 @@ inline SortPlan sort_plan_of(const SortPlanMem& m, int max_tiles) {
 bool sort_plan_fits(int64_t max_tiles);   // the sort's counts of so many tiles are numbered in 31 bits
 
 // Builds the plan on the device from segment boundaries offsets[s * stride], s = 0..num_segments
-// (int32 or int64, clamped to [0, n]) into plan_mem. One small kernel, no host read. Boundaries that
+// (int32 or int64, clamped to [0, n]) into plan_mem. One small kernel or two, no host read. Boundaries that
 // decrease raise B200TBE_DEV_OFFSETS_NOT_MONOTONE in *status, and the plan then has no tiles.
 int build_sort_plan(const void* offsets, int offset_bytes, int num_segments, int64_t stride, int64_t n,
                     void* plan_mem, int32_t* status, SortPlan* plan, cudaStream_t stream);

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kBwdThreads)
                           const SortPlanMem plan, int max_tiles, uint8_t* __restrict__ flags, int64_t num_flags,
                           bool all_flags) {
   if (blockIdx.x == 0) {
-    plan_sort(p.offsets, static_cast<int>(sizeof(IndexT)), p.T, p.B, p.num_indices, max_tiles, plan, p.status);
+    plan_sort<kBwdThreads, 4, true>(p.offsets, static_cast<int>(sizeof(IndexT)), p.T, p.B, p.num_indices, max_tiles, plan, p.status);
     return;
   }
   const int lane = threadIdx.x & 31;
