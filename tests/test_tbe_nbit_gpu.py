@@ -220,3 +220,23 @@ def test_nbit_weights_that_are_not_finite_stay_in_their_bags(D, align, B):
         clean = ~touched[t * B:(t + 1) * B]
         # sums of at most 70 dequantised terms of magnitude <= 1.5, in another order
         np.testing.assert_allclose(got[clean, t * D:(t + 1) * D], want[clean, t * D:(t + 1) * D], rtol=1e-5, atol=3e-5)
+
+
+@pytest.mark.parametrize("T", [2, 31, 33, 64, 129, 1023, 1024, 1025, 2100])
+@pytest.mark.parametrize("types", ["alternating", "one_int8", "one_int4", "random"])
+def test_nbit_tables_of_both_types_at_every_count(T, types):
+    """Grids of more than one wave take INT8 tables before the others: every table is pooled once, wherever its type
+    puts it."""
+    rng = workloads.rng_for(370 + T)
+    ty = {"alternating": np.arange(T) % 2, "one_int8": (np.arange(T) != T - 1).astype(int),
+          "one_int4": (np.arange(T) == T // 2).astype(int), "random": rng.integers(0, 2, size=T)}[types]
+    tys = [oracle.INT4 if x else oracle.INT8 for x in ty]
+    rows, D = 7, 16
+    B = 10_000 // T + 3       # one bag per CTA, more CTAs than run at a time
+    W, wo, Do, tys_a = helpers.quantised_tables(rng, [rows] * T, [D] * T, tys, 16)
+    _, offsets, indices = helpers.ragged_bags(rng, T, B, [rows] * T, 0, 3)
+    want = oracle.nbit_forward(W, wo, tys_a, Do, 16, B, indices, offsets)
+    for tell in (True, False):
+        got, status = _run(W, wo, tys_a, Do, [rows] * T, B, indices, offsets, None, oracle.SUM, torch.float32, 16, tell)
+        assert status == 0
+        np.testing.assert_allclose(got.cpu().numpy(), want, rtol=1e-5, atol=1e-5)

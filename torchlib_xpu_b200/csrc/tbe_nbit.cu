@@ -153,6 +153,7 @@ int launch_bags(const NbitParams& d0, cudaStream_t stream) {
   d.bag_group = bag_group_for(bags) < 8 ? bag_group_for(bags) : 8;
   d.groups_per_table = (d.B + d.bag_group - 1) / d.bag_group;
   const int64_t ctas = static_cast<int64_t>(d.T) * d.groups_per_table;
+  d.by_type = d.by_type && ctas > int64_t{kNumSMs} * kNbitBagCtasPerSm;   // all in flight at once: no order to speak of
   if (d.per_sample_weights != nullptr)
     tbe_nbit_bags_kernel<OT, IndexT, true><<<static_cast<unsigned>(ctas), kNbitBagThreads, 0, stream>>>(d);
   else
@@ -217,9 +218,11 @@ extern "C" int b200tbe_nbit_forward(const b200tbe_nbit_forward_params* p,
   // types present, when the caller says (bit i: some table has type code i): with INT8 and INT4
   // alone and narrow rows the ring kernel would find nothing to do and is not launched
   const uint32_t fast_types = (1u << B200TBE_INT8) | (1u << B200TBE_INT4);
-  // INT8 beside INT4 or types unknown (one type alone needs no order)
-  d.by_type = p->T > 1 && p->T <= kNbitOrderedTables &&
-              (p->table_type_mask == 0 || (p->table_type_mask & fast_types) == fast_types);
+  // INT8 beside INT4 or types unknown (one type alone needs no order). Places among more tables cost more, and are
+  // worth it where the loops are long: 160 alternating tables take 564 us without and 290 with an order at D = 128,
+  // but 200 and 206 at D = 64, and weighted rows of D = 128, whose loops are shorter, 334 and 337.
+  d.by_type = p->T > 1 && (p->table_type_mask == 0 || (p->table_type_mask & fast_types) == fast_types) &&
+              (p->T <= kNbitWordTables || (p->per_sample_weights == nullptr && p->max_D > 64));
   d.only_bag_tables = p->table_type_mask != 0 && (p->table_type_mask & ~fast_types) == 0 &&
                       p->max_D <= kNbitBagMaxD && p->row_alignment % 4 == 0;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);

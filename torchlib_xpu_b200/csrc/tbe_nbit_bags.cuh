@@ -594,10 +594,11 @@ __device__ __forceinline__ void pool_quantised_vector_table(const NbitParams& p,
 
 // The table at place `place` when INT8 tables come first and all others after them, both in their order. The
 // loops for INT8 and INT4 rows do not fit the instruction cache together: with tables of both types in
-// flight on every SM the call took up to twice as long as one type after the other. One warp, all lanes.
-constexpr int kNbitOrderedTables = 128;   // beyond that the places cost more loads than they are worth
-__device__ __forceinline__ int table_by_type(const uint8_t* __restrict__ tys, int T, int place, int lane) {
-  constexpr int kWords = kNbitOrderedTables / 32;
+// flight on every SM the call takes up to twice as long as one type after the other (129 / 512 / 1024 alternating
+// tables, D = 128: 457 / 456 / 461 us without an order, 245 / 249 / 257 with it). One warp, all lanes.
+constexpr int kNbitWordTables = 128;   // as many types are held as four words
+__device__ __forceinline__ int table_by_type_of_few(const uint8_t* __restrict__ tys, int T, int place, int lane) {
+  constexpr int kWords = kNbitWordTables / 32;
   uint32_t int8[kWords];
   int count8 = 0;
 #pragma unroll
@@ -620,6 +621,57 @@ __device__ __forceinline__ int table_by_type(const uint8_t* __restrict__ tys, in
     nth -= __popc(mask);
   }
   return found;
+}
+
+// Any number of tables: lane i holds the types of tables 32 i .. 32 i + 31 of a block of 1024 as bits. (Out of line:
+// inlined, it moves the loops of weighted 32-element rows in the kernel, 172 -> 180 us for 160 tables without an order.)
+__device__ __noinline__ int table_by_type_of_many(const uint8_t* __restrict__ tys, int T, int place, int lane) {
+  auto int8_tables = [&](int base) {
+    const int words = T - base < 1024 ? (T - base + 31) >> 5 : 32;
+    uint32_t mine = 0;
+#pragma unroll 4
+    for (int i = 0; i < words; ++i) {
+      const int t = base + 32 * i + lane;
+      const uint32_t mask = __ballot_sync(kFullMask, t < T && __ldg(tys + t) == B200TBE_INT8);
+      if (lane == i) mine = mask;
+    }
+    return mine;
+  };
+  uint32_t mine = 0;
+  int count8 = 0;
+  for (int base = 0; base < T; base += 1024) {
+    mine = int8_tables(base);
+    count8 += static_cast<int>(__reduce_add_sync(kFullMask, static_cast<unsigned>(__popc(mine))));
+  }
+  const bool first = place < count8;
+  int nth = first ? place : place - count8;   // the nth table of its kind
+  for (int base = 0; base < T; base += 1024) {
+    if (T > 1024) mine = int8_tables(base);
+    const int left = T - base - 32 * lane;
+    const uint32_t all = left >= 32 ? kFullMask : (left > 0 ? (1u << left) - 1u : 0u);
+    const uint32_t mask = (first ? mine : ~mine) & all;
+    const int here = __popc(mask);
+    int upto = here;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int below = __shfl_up_sync(kFullMask, upto, o);
+      if (lane >= o) upto += below;
+    }
+    const uint32_t hit = __ballot_sync(kFullMask, upto > nth);
+    if (hit != 0) {
+      const int word = __ffs(hit) - 1;
+      const uint32_t bits = __shfl_sync(kFullMask, mask, word);
+      const int rest = nth - __shfl_sync(kFullMask, upto - here, word);
+      const bool me = ((bits >> lane) & 1u) && __popc(bits & ((1u << lane) - 1u)) == rest;
+      return base + 32 * word + __ffs(__ballot_sync(kFullMask, me)) - 1;
+    }
+    nth -= __shfl_sync(kFullMask, upto, 31);
+  }
+  return 0;
+}
+
+__device__ __forceinline__ int table_by_type(const uint8_t* __restrict__ tys, int T, int place, int lane) {
+  return T <= kNbitWordTables ? table_by_type_of_few(tys, T, place, lane) : table_by_type_of_many(tys, T, place, lane);
 }
 
 template <typename OT, typename IndexT, bool kWeighted>
