@@ -314,3 +314,27 @@ def test_forward_weights_that_are_not_finite_stay_in_their_bags(wdtype, Ds, idx_
         np.testing.assert_allclose(got[clean, Do[t]:Do[t + 1]], want[clean, Do[t]:Do[t + 1]], rtol=RTOL_FP32,
                                    atol=1.5 * ATOL_FP32_UNIT)
         assert not np.isfinite(got[~clean, Do[t]:Do[t + 1]]).any()
+
+
+@pytest.mark.parametrize("wdtype,Ds", [(np.float32, (260, 512, 64)), (np.float16, (1024, 264, 128))])
+@pytest.mark.parametrize("B,rpd", [(40, 14), (16_003, 5_335)])      # one bag per warp, groups of bags
+@pytest.mark.parametrize("col0,extra", [(8, 8), (3, 2)])            # aligned and unaligned output rows
+def test_forward_wide_rows_across_destinations(wdtype, Ds, B, rpd, col0, extra):
+    """Rows of 513 to 2048 bytes with num_dests > 1: a destination's last row falls inside a group of bags."""
+    rng = workloads.rng_for(250 + sum(Ds))
+    rows, T, G = [60, 300, 20], len(Ds), 3
+    W, wo, Do = helpers.float_tables(rng, rows, Ds, wdtype, -1.0, 1.0)
+    _, offsets, indices = helpers.ragged_bags(rng, T, B, rows, 0, 5, empty_fraction=0.2)
+    ty = oracle.FP32 if wdtype == np.float32 else oracle.FP16
+    want = oracle.tbe_forward(W, ty, wo, Do, B, indices, offsets)
+    total_D = int(Do[-1])
+    stride = col0 + total_D + extra
+    bufs = [torch.full((rpd, stride), -7.0, dtype=torch.float32, device="cuda") for _ in range(G)]
+    cabi.forward(_dev(W), _dev(wo), _dev(Do), total_D, max(Ds), _dev(indices), _dev(offsets), B, outputs=bufs,
+                 output_stride=stride, output_col_offset=col0, rows_per_dest=rpd, output_dtype=torch.float32)
+    torch.cuda.synchronize()
+    for g, buf in enumerate(bufs):
+        blk = buf.cpu().numpy()
+        n = min(rpd, B - g * rpd)
+        np.testing.assert_allclose(blk[:n, col0:col0 + total_D], want[g * rpd:g * rpd + n], rtol=RTOL_FP32, atol=ATOL_FP32_UNIT)
+        assert np.all(blk[:, :col0] == -7.0) and np.all(blk[:, col0 + total_D:] == -7.0) and np.all(blk[n:] == -7.0)

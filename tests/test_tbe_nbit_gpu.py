@@ -1,4 +1,6 @@
 """GPU parity: quantised-inference TBE forward through the C ABI vs the CPU oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -240,3 +242,36 @@ def test_nbit_tables_of_both_types_at_every_count(T, types):
         got, status = _run(W, wo, tys_a, Do, [rows] * T, B, indices, offsets, None, oracle.SUM, torch.float32, 16, tell)
         assert status == 0
         np.testing.assert_allclose(got.cpu().numpy(), want, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("Ds,align", [((128, 64, 32), 16), ((512, 256, 16), 16), ((128, 40, 64), 4)])
+@pytest.mark.parametrize("B,rpd", [(40, 14), (16_003, 5_335)])      # one bag per warp, groups of bags
+@pytest.mark.parametrize("out_dtype,col0,extra", [(torch.float16, 8, 8), (torch.float16, 3, 2), (torch.float32, 1, 2)])
+def test_nbit_across_destinations(Ds, align, B, rpd, out_dtype, col0, extra):
+    """num_dests > 1, rows fetched as vectors and as words: a destination's last row falls inside a group of bags;
+    aligned and unaligned output rows."""
+    rng = workloads.rng_for(380 + sum(Ds))
+    tys, rows, T, G = [oracle.INT8, oracle.INT4, oracle.INT4], [60, 300, 20], 3, 3
+    if Ds[1] == 40:
+        tys = [oracle.INT8, oracle.INT4, oracle.INT8]
+    W, wo, Do, tys_a = helpers.quantised_tables(rng, rows, Ds, tys, align)
+    _, offsets, indices = helpers.ragged_bags(rng, T, B, rows, 0, 5, empty_fraction=0.2)
+    want = oracle.nbit_forward(W, wo, tys_a, Do, align, B, indices, offsets)
+    total_D = int(Do[-1])
+    stride = col0 + total_D + extra
+    bufs = [torch.full((rpd, stride), -7.0, dtype=out_dtype, device="cuda") for _ in range(G)]
+    held = [_dev(a) for a in (W, wo, tys_a, Do, indices, offsets)]
+    p = cabi.NbitForwardParams()
+    p.dev_weights, p.weights_offsets, p.weights_tys, p.D_offsets, p.indices, p.offsets = (a.data_ptr() for a in held)
+    for g in range(G):
+        p.outputs[g] = bufs[g].data_ptr()
+    p.output_stride, p.output_col_offset, p.rows_per_dest, p.num_dests = stride, col0, rpd, G
+    p.T, p.B, p.max_D, p.row_alignment, p.index_bytes = T, B, max(Ds), align, 8
+    p.output_dtype, p.pooling_mode = cabi.FP16 if out_dtype == torch.float16 else cabi.FP32, oracle.SUM
+    assert cabi.lib().b200tbe_nbit_forward(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    for g, buf in enumerate(bufs):
+        blk = buf.float().cpu().numpy()
+        n = min(rpd, B - g * rpd)
+        np.testing.assert_allclose(blk[:n, col0:col0 + total_D], want[g * rpd:g * rpd + n], rtol=RTOL, atol=ATOL)
+        assert np.all(blk[:, :col0] == -7.0) and np.all(blk[:, col0 + total_D:] == -7.0) and np.all(blk[n:] == -7.0)
