@@ -210,12 +210,14 @@ def uniform_half_table(num_elems, lo, hi, gen):
     return w
 
 
-def backward_launches(row_bits: int) -> int:
-    """Kernels one b200tbe_backward call of a million lookups or more launches for rows of at most 512
-    elements: linearize (with the plan), per sort pass (8 bits each) histogram + 3 scan kernels + scatter,
-    sweep, finish."""
+def backward_launches(lookups: int, tables: int, row_bits: int) -> int:
+    """Kernels one b200tbe_backward call launches for rows of at most 512 elements: sweep and finish after, in
+    small batches, one kernel that plans, linearises and sorts, else linearise (with the plan) and per sort pass
+    (8 bits each) histogram + scatter, with three scan kernels between them from 257 whole tiles of 4096 on."""
+    if lookups <= 65536 and tables <= 128:
+        return 3
     passes = (row_bits + 7) // 8
-    return 1 + passes * 5 + 2
+    return 1 + passes * (2 if lookups // 4096 <= 256 else 5) + 2
 
 
 def time_launches(fn, iters, flush=None):
@@ -304,7 +306,7 @@ class ShardedTbeStep:
 
     def launches_per_step(self):
         extra = 0 if self.exchange is None else self.exchange.launches_per_step()
-        return 1 + backward_launches(max(1, (self.E - 1).bit_length())) + extra
+        return 1 + backward_launches(self.N, self.T, max(1, (self.E - 1).bit_length())) + extra
 
     def fwd_bytes(self):
         return workloads.forward_bytes(self.N, self.U, self.D * 2, self.T, self.B, self.D, 2)
@@ -469,7 +471,7 @@ def _bench_train(entry, flush, gen, iters):
           inp.num_lookups, {"unique_rows": U})
     ms, _ = time_launches(bwd, iters, flush)
     entry("tbe_fp16_backward_adagrad(config3)", workloads.backward_bytes(inp.num_lookups, U, D * 2, T, B, D, 4),
-          ms, inp.num_lookups, {"kernels_per_call": backward_launches((E - 1).bit_length())})
+          ms, inp.num_lookups, {"kernels_per_call": backward_launches(inp.num_lookups, T, (E - 1).bit_length())})
 
 
 def _bench_uniform(entry, flush, gen, iters):
@@ -501,7 +503,7 @@ def _bench_uniform(entry, flush, gen, iters):
           {"unique_rows": U})
     ms, _ = time_launches(bwd, max(5, iters // 2), flush)
     entry("tbe_fp16_backward_adagrad(uniform ids, 16 GB of rows)", workloads.backward_bytes(n, U, D * 2, T, B, D, 2),
-          ms, n, {"unique_rows": U, "kernels_per_call": backward_launches((E - 1).bit_length())})
+          ms, n, {"unique_rows": U, "kernels_per_call": backward_launches(n, T, (E - 1).bit_length())})
     del W, mom, idx, grad, scratch, out
     # the same lookup on rows of 128 and 64 bytes (D = 64, 32): random rows this short are no longer bound
     # by bytes but by how many rows a second HBM serves, which is what the quantised tables' rows meet
