@@ -214,7 +214,7 @@ def backward_launches(lookups: int, tables: int, row_bits: int) -> int:
     """Kernels one b200tbe_backward call launches for rows of at most 512 elements: sweep and finish after, in
     small batches, one kernel that plans, linearises and sorts, else linearise (with the plan) and per sort pass
     (8 bits each) histogram + scatter, with three scan kernels between them from 257 whole tiles of 4096 on."""
-    if lookups <= 65536 and tables <= 128:
+    if lookups <= 65536 and tables <= 96:
         return 3
     passes = (row_bits + 7) // 8
     return 1 + passes * (2 if lookups // 4096 <= 256 else 5) + 2

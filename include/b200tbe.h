@@ -62,7 +62,7 @@ typedef enum { B200TBE_OPT_SGD = 0, B200TBE_OPT_ROWWISE_ADAGRAD = 1 } b200tbe_op
 /* Bits a kernel may OR into the optional device status word (int32). */
 #define B200TBE_DEV_INDEX_OUT_OF_RANGE 1
 /* b200tbe_backward found offsets that decrease; it has changed nothing. Found: any table that ends before it
- * begins; any bag that does, from 65 537 lookups on, beyond 128 tables and for rows of more than 512 elements
+ * begins; any bag that does, from 65 537 lookups on, beyond 96 tables and for rows of more than 512 elements
  * (in smaller batches such a bag only moves lookups of its table to other bags of the table). */
 #define B200TBE_DEV_OFFSETS_NOT_MONOTONE 2
 #define B200TBE_DEV_UNSUPPORTED_SHAPE 4 /* a table's row is not whole 16-byte vectors */
@@ -338,10 +338,11 @@ B200TBE_API int b200tbe_permute_segments(const void* in, void* out, const void* 
  * b200tbe_permute_row_starts writes in_start[out_rows] (where output row j's elements begin in the
  * input), out_offsets[out_rows + 1] (where they begin in the output) and, when permuted_lengths is
  * not null, the permuted [out_rows][cols] lengths. A perm entry outside [0, rows) fails a device
- * assertion.
+ * assertion where the lengths are permuted too; where permuted_lengths is null it stands for an empty
+ * row.
  * b200tbe_permute_rows moves one array of elem_bytes-wide elements (2, 4 or 8) and, when in2 is not
- * null, a second one of elem2_bytes (ids and their per-sample weights: one launch for 8- or 4-byte
- * elements with 4-byte ones). Output elements past out_offsets[out_rows] are left as they are.
+ * null, a second one of elem2_bytes, 2, 4 or 8 (ids and their per-sample weights: one launch for 8- or
+ * 4-byte elements with 4-byte ones); any other width is refused before anything is moved. Output elements past out_offsets[out_rows] are left as they are.
  * ---------------------------------------------------------------------------------------------- */
 B200TBE_API size_t b200tbe_permute_row_starts_scratch_bytes(int64_t rows, int64_t cols);
 B200TBE_API int b200tbe_permute_row_starts(const void* lengths, const void* perm, void* permuted_lengths,

@@ -563,3 +563,10 @@ def test_backward_over_many_tables(T, B):
     rows, Ds = [60] * T, [8] * T
     case = _backward_case(rng, rows, Ds, B, 0, 14, np.float32, np.float32, oracle.SUM, oracle.SGD, False)
     _check(*case, B, np.float32, np.float32, oracle.SUM, oracle.SGD)
+
+
+@pytest.mark.parametrize("T", [96, 97])
+def test_backward_small_batch_at_the_most_tables_of_one_launch(T):
+    rng = workloads.rng_for(492)
+    case = _backward_case(rng, [60] * T, [8] * T, 9, 0, 6, np.float32, np.float32, oracle.SUM, oracle.ROWWISE_ADAGRAD, True)
+    _check(*case, 9, np.float32, np.float32, oracle.SUM, oracle.ROWWISE_ADAGRAD)

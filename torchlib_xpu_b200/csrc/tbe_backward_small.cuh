@@ -1,9 +1,9 @@
 // Plan, linearise and sort of a small batch (at most kSmallSortMax lookups) in one launch.
 //
-// The general path takes 18 launches of 2 to 7 us for this, whatever the batch: 8 tables x 256 samples
-// (11 000 lookups) spent 85 us between the forward and the sweep, 14 us here (60 000 lookups of two tables:
-// 34 us, still half of the general path). One cluster of
-// eight CTAs sorts one table: every CTA holds an eighth of the table's lookups in registers (whatever the
+// The general path takes seven launches of 2 to 7 us for this (linearise with the plan, histogram and scatter for
+// each of three passes) with gaps between them: 8 tables x 256 samples (11 000 lookups) spend 28 us in its kernels and
+// 15 us in this one, a training step 112 and 90 us; 60 000 lookups of two tables 35 us either way, a step 95 and 91.
+// One cluster of eight CTAs sorts one table: every CTA holds an eighth of the table's lookups in registers (whatever the
 // distribution over the tables, a table's lookups fit a cluster), and per pass of up to 8 bits
 //   * ranks its keys by digit, warp by warp (one vote per digit bit, as in radix_sort.cu),
 //   * reads the other seven CTAs' digit counts out of their shared memory, and
@@ -20,9 +20,10 @@ constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kSmallItems = 16;                                       // keys per thread
 constexpr int kSmallCluster = 8;                                      // CTAs per table
 constexpr int kSmallSortMax = kSmallCluster * kSmallThreads * kSmallItems;   // 65536
-// A table takes a cluster however few lookups it has, and some 37 clusters run at a time: 41 000 lookups over
-// 32 / 64 / 128 tables take 13 / 26 / 49 us, the general path's seven launches about 50.
-constexpr int kSmallSortTables = 128;
+// A table takes a cluster however few lookups it has, and some 37 clusters run at a time: training steps of 41 000
+// lookups over 32 / 64 / 80 / 96 / 112 / 128 tables take 91 / 82 / 86 / 92 / 104 / 109 us this way (the kernel 14 / 26 /
+// - / - / - / 49) and 101 / 94 / 95 / 95 / 93 / 94 by the general path.
+constexpr int kSmallSortTables = 96;
 constexpr int kSmallRadix = 256;
 constexpr int kSmallBags = 4096;                                      // bag starts kept in shared memory
 
