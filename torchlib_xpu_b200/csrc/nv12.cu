@@ -146,8 +146,10 @@ __device__ __forceinline__ void convert_row16(const LumaScale& ls, const LumaSca
   out[2] = make_uint4(w[8], w[9], w[10], w[11]);
 }
 
-// A plain grid, one block of 16 pixels x 2 rows per thread, no shared memory. Eight CTAs per SM (32
-// registers): a 4K frame is 1013 CTAs, one wave instead of one and a bit (12.31 -> 12.29 us a call).
+// A plain grid, one block of 16 pixels x 2 rows per thread, no shared memory. Eight CTAs per SM (32 registers, four
+// bytes spilled): a 4K frame is 1013 CTAs, one wave instead of one and a bit, which is what a frame that is not in L2
+// waits for: 14.3 us instead of 16.4 without the bound (40 registers), 32 such frames 0.398 instead of 0.413 ms.
+// Frames that are in L2 take 2.83 / 4.36 / 9.87 us (640 x 360 / 1920 x 1080 / 3840 x 2160) instead of 2.71 / 4.29 / 9.71.
 __global__ void __launch_bounds__(kNv12Threads, 8)
     nv12_to_rgb_blocks_kernel(const uint8_t* __restrict__ y_plane, const uint8_t* __restrict__ uv_plane,
                               uint8_t* __restrict__ rgb, int width, int height, int stride,
